@@ -10,19 +10,27 @@
 // broken lexicographically, scanning the variants in the reference's order; the
 // configuration's hash code is that hash.
 //
-// Per warp and row: the spi cycle tables (leader = smallest symbol, t = forward steps from
-// the leader, L) go to shared memory once.  Per variant, each lane takes pi positions
-// p = lane and lane + 32:
-//  * its symbol's cycle in the variant (the mirror runs spi's cycles backwards through the
-//    involution), the cycle's first position along pi (shared-memory atomicMin per cycle),
-//    label = rank of that first position among the cycles' first positions, orientation =
-//    more than one leap of pi^-1 positions around the cycle (atomicAdd per cycle), index of
-//    an oriented symbol along the cycle from the symbol at the cycle's first position.
-// Variants are built 32 at a time into a shared-memory block of rows; then the lanes switch to
-// variants and each computes its row's CRC32 from a byte table.  The least hash, ties broken
-// by the lexicographically least row, does not depend on the order the variants are
-// scanned in, so the groups give the reference's answer.  The best row so far stays in
-// shared memory.
+// One warp per row, lanes over variants.  What makes a lane's walk along its variant cheap:
+//  * whether a cycle is oriented (more than one leap of pi^-1 positions) is the same in every
+//    variant: with d = (pos(succ) - pos(s)) mod n, the descents around a cycle number
+//    sum(d) / n, and neither a rotation of pi nor the mirror changes a d.  So the cycle tables
+//    (cycle number, steps t from the least symbol, length, orientation) are built once per row.
+//  * the walk needs no positions: the label of a cycle is the count of cycles met before it,
+//    plus one, and the index of an oriented symbol is t minus the t of the cycle's first symbol
+//    met (modulo its length; the mirror runs t backwards).  Each lane keeps (label, first t)
+//    per cycle in its own column of shared memory.
+//  * the CRC32 takes a whole float per step: crc' is linear in crc ^ value, so it is the xor of
+//    seven table entries selected by 5-bit windows.  A window's table has 32 words, one per
+//    bank, so the lookups of a warp never conflict (a byte table costs about 3.5 wavefronts per
+//    lookup, and four of them in series per float).
+// The least hash is reduced over lanes and groups of 32 variants.  Only the winner's row is
+// written out, built position-parallel; variants that tie with it on the hash (mostly
+// symmetric configurations, with equal rows) are built and compared the same way, in variant
+// order.
+// Bound: instruction issue (about 45 instructions per variant and position) and the shared
+// memory pipe (11 wavefronts); HBM moves 329 bytes per row.  250,000 rows of 3..10 3-cycles
+// on one B200: 2,780 us with lanes over positions, shared-memory atomics per variant and a byte
+// table per CRC; NEW_US us in this form.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -34,8 +42,8 @@
 namespace tdp {
 namespace {
 
-constexpr int kWarps = 4;   // warps (configurations) per block
-constexpr int kMaxN = 63;   // two pi positions per lane
+constexpr int kWarps = 8;   // warps (configurations) per block
+constexpr int kMaxN = 63;   // two symbols per lane in the position-parallel parts; at most 31 cycles
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr uint32_t kPoly = 0xEDB88320u;  // reflected CRC-32 polynomial (java.util.zip.CRC32)
 
@@ -48,25 +56,79 @@ struct CanonArgs {
     int32_t *variant;
 };
 
-constexpr int kRowPitch = 65;  // floats per row: an odd pitch keeps variant-major reads off one bank
+// A symbol's word: cycle number << 7 (the byte offset of its row in WarpSmem::met), t, length
+// and orientation; t, length and the orientation bit are 0 on unoriented cycles.
+constexpr uint32_t kCycleOffset = 31u << 7;
+constexpr int kTShift = 12, kLenShift = 18, kOrientedShift = 24;
 
 struct WarpSmem {
-    float rows[32][kRowPitch];  // the current group of up to 32 variant rows
+    uint32_t met[32][32];      // [cycle][lane]: float bits of the label | first t; 0 = not met
+    uint32_t word[2][2 * 64];  // [mirror][symbol], two periods: no wrap along a walk
+    uint8_t spi[64];
     float best[64];
-    uint8_t spi[64], inv[64], leader[64], t[64], len[64];
-    int firstPos[64], leaps[64], anchorT[64], count[64];
+    int firstPos[32], anchor[32];
 };
 
-__device__ __forceinline__ int mod_n(int x, int n) { return x >= n ? x - n : (x < 0 ? x + n : x); }
+// The signature value of one symbol: label plus index/100 (index 0 on unoriented cycles), the
+// same two single-precision operations as Java's label + (float) index / 100.
+__device__ __forceinline__ float value_of(const float *hundredth, uint32_t w, uint32_t met) {
+    int idx = (int)((w >> kTShift) & 63u) - (int)(met & 63u);
+    if (idx < 0) idx += (int)((w >> kLenShift) & 63u);
+    return __fadd_rn(__uint_as_float(met & ~63u), hundredth[idx + (int)(w >> kOrientedShift)]);
+}
+
+// The row of one variant, lanes over positions: value at positions lane and lane + 32.
+__device__ __forceinline__ void build_row(WarpSmem &S, const float *hundredth, int variant, int n, int lane,
+                                          float (&value)[2]) {
+    const int r = variant >> 1, mirror = variant & 1;
+    S.firstPos[lane] = 127;
+    __syncwarp();
+    uint32_t w[2];
+    int cycle[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int p = lane + 32 * h;
+        w[h] = 0u, cycle[h] = 0;
+        if (p < n) {
+            w[h] = S.word[mirror][mirror ? r + n - 1 - p : r + p];
+            cycle[h] = (int)((w[h] & kCycleOffset) >> 7);
+            atomicMin(&S.firstPos[cycle[h]], p);
+        }
+    }
+    __syncwarp();
+    bool first[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int p = lane + 32 * h;
+        first[h] = p < n && S.firstPos[cycle[h]] == p;
+        if (first[h]) S.anchor[cycle[h]] = (int)((w[h] >> kTShift) & 63u);
+    }
+    const uint64_t firsts =
+        (uint64_t)__ballot_sync(kFull, first[0]) | ((uint64_t)__ballot_sync(kFull, first[1]) << 32);
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        value[h] = 0.f;
+        if (lane + 32 * h < n) {
+            const int fp = S.firstPos[cycle[h]];
+            const int label = __popcll(firsts & ((2ull << fp) - 1ull));
+            value[h] = value_of(hundredth, w[h],
+                                __float_as_uint(__int2float_rn(label)) | (uint32_t)S.anchor[cycle[h]]);
+        }
+    }
+    __syncwarp();
+}
 
 __global__ void __launch_bounds__(kWarps * 32) canonical_kernel(const CanonArgs A) {
-    __shared__ uint32_t crcTable[256];
+    __shared__ uint32_t crc5[7][32];    // crc5[k][e]: 32 CRC steps on e << 5k
+    __shared__ float hundredth[64];     // i / 100, and 0 for unoriented symbols
     __shared__ WarpSmem smem[kWarps];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        uint32_t c = (uint32_t)i;
-        for (int k = 0; k < 8; ++k) c = (c >> 1) ^ (kPoly & (0u - (c & 1u)));
-        crcTable[i] = c;
+    for (int i = threadIdx.x; i < 7 * 32; i += blockDim.x) {
+        uint32_t c = (i >> 5) < 6 ? (uint32_t)(i & 31) << (5 * (i >> 5)) : (uint32_t)(i & 3) << 30;
+        for (int k = 0; k < 32; ++k) c = (c >> 1) ^ (kPoly & (0u - (c & 1u)));
+        crc5[i >> 5][i & 31] = c;
     }
+    if (threadIdx.x < 64) hundredth[threadIdx.x] = __fdiv_rn(__int2float_rn((int)threadIdx.x), 100.0f);
     __syncthreads();
     const int lane = threadIdx.x & 31;
     WarpSmem &S = smem[threadIdx.x >> 5];
@@ -75,36 +137,23 @@ __global__ void __launch_bounds__(kWarps * 32) canonical_kernel(const CanonArgs 
         const uint8_t *src = A.spi + (size_t)row * 64;
         // validity: 2 <= n <= 63, spi a permutation of 0..n-1 without fixed points; a bad row
         // gets variant -1, hash 0 and a zero signature
-        S.count[lane] = 0;
-        S.count[lane + 32] = 0;
-        __syncwarp();
         bool bad = n < 2 || n > kMaxN;
+        uint32_t seen[2] = {0u, 0u};
         if (!bad) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int x = lane + 32 * h;
                 if (x < n) {
                     const int s = src[x];
-                    if (s >= n || s == x) {
-                        bad = true;
-                    } else {
-                        atomicAdd(&S.count[s], 1);
-                        S.spi[x] = (uint8_t)s;
-                        S.inv[s] = (uint8_t)x;
-                    }
+                    bad |= s >= n || s == x;
+                    seen[(s >> 5) & 1] |= 1u << (s & 31);
+                    S.spi[x] = (uint8_t)s;
                 }
             }
         }
-        __syncwarp();
-        if (!bad) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int x = lane + 32 * h;
-                if (x < n && S.count[x] != 1) bad = true;
-            }
-        }
+        const int distinct = __popc(__reduce_or_sync(kFull, seen[0])) + __popc(__reduce_or_sync(kFull, seen[1]));
         float *dst = A.sig + (size_t)row * 64;
-        if (__any_sync(kFull, bad)) {
+        if (__any_sync(kFull, bad || distinct != n)) {
             dst[lane] = 0.f;
             dst[lane + 32] = 0.f;
             if (lane == 0) {
@@ -114,135 +163,124 @@ __global__ void __launch_bounds__(kWarps * 32) canonical_kernel(const CanonArgs 
             __syncwarp();
             continue;
         }
-        // spi cycle tables: each lane walks the cycles of its symbols (length <= n)
+        __syncwarp();
+        // cycle tables: each lane walks the cycles of its symbols (length <= n)
+        int least[2], t[2], len[2], ascents[2];
+        bool leads[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int x = lane + 32 * h;
+            least[h] = x, t[h] = 0, len[h] = 1, ascents[h] = 0;
+            if (x < n) {
+                int at = 0, prev = x;
+                for (int y = S.spi[x]; y != x && len[h] <= kMaxN; y = S.spi[y]) {
+                    if (y < least[h]) least[h] = y, at = len[h];
+                    ascents[h] += prev < y ? 1 : 0;
+                    prev = y;
+                    ++len[h];
+                }
+                ascents[h] += prev < x ? 1 : 0;
+                t[h] = at == 0 ? 0 : len[h] - at;
+            }
+            leads[h] = x < n && least[h] == x;
+        }
+        const uint64_t leaders =
+            (uint64_t)__ballot_sync(kFull, leads[0]) | ((uint64_t)__ballot_sync(kFull, leads[1]) << 32);
+        const int cycles = __popcll(leaders);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int x = lane + 32 * h;
             if (x < n) {
-                int m = x, steps = 0, L = 1;
-                for (int y = S.spi[x]; y != x && L <= kMaxN; y = S.spi[y]) {
-                    m = min(m, y);
-                    ++L;
+                const uint32_t cycle = (uint32_t)__popcll(leaders & ((1ull << least[h]) - 1ull)) << 7;
+                uint32_t fwd = cycle, mir = cycle;
+                if (ascents[h] > 1) {
+                    const uint32_t rest = ((uint32_t)len[h] << kLenShift) | (1u << kOrientedShift);
+                    fwd |= rest | ((uint32_t)t[h] << kTShift);
+                    // the mirror runs spi's cycle backwards
+                    mir |= rest | ((uint32_t)(t[h] == 0 ? 0 : len[h] - t[h]) << kTShift);
                 }
-                for (int y = x; y != m && steps <= kMaxN; y = S.spi[y]) ++steps;
-                S.leader[x] = (uint8_t)m;
-                S.t[x] = (uint8_t)(steps == 0 ? 0 : L - steps);
-                S.len[x] = (uint8_t)L;
+                S.word[0][x] = S.word[0][x + n] = fwd;
+                S.word[1][x] = S.word[1][x + n] = mir;
             }
         }
         __syncwarp();
-        int32_t bestHash = INT32_MAX;
-        int bestV = -1;
-        for (int group = 0; group < 2 * n; group += 32) {
-            const int nv = min(32, 2 * n - group);
-            for (int k = 0; k < nv; ++k) {
-                const int v = group + k;
-                const int r = v >> 1;
-                const bool mirror = v & 1;
-                S.firstPos[lane] = 127;
-                S.firstPos[lane + 32] = 127;
-                S.leaps[lane] = 0;
-                S.leaps[lane + 32] = 0;
-                __syncwarp();
-                int cid[2], tS[2], L[2];
-                bool act[2];
+        // slot u < n: pi started at u; slot n + u: its mirror.  Slots go to lanes 32 at a time.
+        int32_t hash[4];
+        const int groups = (2 * n + 31) >> 5;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int p = lane + 32 * h;
-                    act[h] = p < n;
-                    cid[h] = 0, tS[h] = 0, L[h] = 1;
-                    if (act[h]) {
-                        const int s = mod_n(r + p, n);
-                        int succ;
-                        if (!mirror) {
-                            succ = S.spi[s];
-                            cid[h] = S.leader[s];
-                            tS[h] = S.t[s];
-                            L[h] = S.len[s];
-                        } else {
-                            // c(x) = symbol at pi position n-1-pos(x); m(x) = c(spi^-1(c(x)))
-                            const int cs = mod_n(r + (n - 1 - p), n);
-                            const int pp = mod_n((int)S.inv[cs] - r, n);
-                            succ = mod_n(r + (n - 1 - pp), n);
-                            cid[h] = S.leader[cs];
-                            L[h] = S.len[cs];
-                            tS[h] = S.t[cs] == 0 ? 0 : L[h] - S.t[cs];  // m runs spi's cycle backwards
-                        }
-                        atomicMin(&S.firstPos[cid[h]], p);
-                        // leap of pi^-1 positions: n-1-pos(s) > n-1-pos(succ) <=> pos(s) < pos(succ)
-                        if (p < mod_n(succ - r, n)) atomicAdd(&S.leaps[cid[h]], 1);
-                    }
-                }
-                __syncwarp();
-                bool isFirst[2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    isFirst[h] = act[h] && S.firstPos[cid[h]] == lane + 32 * h;
-                    if (isFirst[h]) S.anchorT[cid[h]] = tS[h];
-                }
-                const uint64_t firsts = (uint64_t)__ballot_sync(kFull, isFirst[0]) |
-                                        ((uint64_t)__ballot_sync(kFull, isFirst[1]) << 32);
-                __syncwarp();
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (act[h]) {
-                        const int fp = S.firstPos[cid[h]];
-                        const uint64_t upTo = (fp >= 63) ? ~0ull : ((2ull << fp) - 1ull);
-                        const int label = __popcll(firsts & upTo);
-                        const bool oriented = S.leaps[cid[h]] > 1;
-                        int idx = tS[h] - S.anchorT[cid[h]];
-                        if (idx < 0) idx += L[h];
-                        const float fl = __int2float_rn(label);
-                        S.rows[k][lane + 32 * h] =
-                            oriented ? __fadd_rn(fl, __fdiv_rn(__int2float_rn(idx + 1), 100.0f)) : fl;
-                    }
-                }
-                __syncwarp();
-            }
-            // lanes = variants of the group: CRC32 of the row's big-endian float bytes
-            int32_t h = INT32_MAX;
-            if (lane < nv) {
+        for (int g = 0; g < 4; ++g) {
+            hash[g] = INT32_MAX;
+            const int u = lane + 32 * g;
+            if (g < groups && u < 2 * n) {
+                const bool mirror = u >= n;
+                const int r = mirror ? u - n : u;
+                const uint32_t *w = mirror ? &S.word[1][r + n - 1] : &S.word[0][r];
+                const int dir = mirror ? -1 : 1;
+                char *const met = reinterpret_cast<char *>(&S.met[0][lane]);
+                for (int c = 0; c < cycles; ++c) *reinterpret_cast<uint32_t *>(met + (c << 7)) = 0u;
+                float labels = 0.f;
                 uint32_t crc = 0xFFFFFFFFu;
-                for (int i = 0; i < n; ++i) {
-                    const uint32_t bits = __float_as_uint(S.rows[lane][i]);
-#pragma unroll
-                    for (int b = 3; b >= 0; --b) crc = crcTable[(crc ^ (bits >> (8 * b))) & 0xFFu] ^ (crc >> 8);
-                }
-                h = (int32_t)(crc ^ 0xFFFFFFFFu);
-            }
-            const int32_t m = __reduce_min_sync(kFull, h);
-            const unsigned cand = __ballot_sync(kFull, lane < nv && h == m);
-            // Configuration.getCanonical: the least hash, ties by Arrays.compare
-            if (lane == 0 && m <= bestHash) {
-                unsigned c = cand;
-                while (c) {
-                    const int w = __ffs(c) - 1;
-                    c &= c - 1u;
-                    bool take = bestV < 0 || m < bestHash;
-                    if (!take) {
-                        for (int i = 0; i < n; ++i) {
-                            const float a = S.rows[w][i], b = S.best[i];
-                            if (a != b) {
-                                take = a < b;
-                                break;
-                            }
-                        }
+#pragma unroll 2
+                for (int p = 0; p < n; ++p, w += dir) {
+                    const uint32_t sym = *w;
+                    uint32_t *const m = reinterpret_cast<uint32_t *>(met + (sym & kCycleOffset));
+                    uint32_t e = *m;
+                    if (e == 0u) {
+                        labels = __fadd_rn(labels, 1.0f);
+                        e = __float_as_uint(labels) | ((sym >> kTShift) & 63u);
+                        *m = e;
                     }
-                    if (take) {
-                        bestHash = m;
-                        bestV = group + w;
-                        for (int i = 0; i < n; ++i) S.best[i] = S.rows[w][i];
-                    }
+                    const uint32_t x =
+                        crc ^ __byte_perm(__float_as_uint(value_of(hundredth, sym, e)), 0u, 0x0123);
+                    crc = crc5[0][x & 31u] ^ crc5[1][(x >> 5) & 31u] ^ crc5[2][(x >> 10) & 31u] ^
+                          crc5[3][(x >> 15) & 31u] ^ crc5[4][(x >> 20) & 31u] ^ crc5[5][(x >> 25) & 31u] ^
+                          crc5[6][x >> 30];
                 }
+                hash[g] = (int32_t)(crc ^ 0xFFFFFFFFu);
             }
-            bestHash = __shfl_sync(kFull, bestHash, 0);
-            bestV = __shfl_sync(kFull, bestV, 0);
-            __syncwarp();
         }
-        dst[lane] = lane < n ? S.best[lane] : 0.f;
-        dst[lane + 32] = lane + 32 < n ? S.best[lane + 32] : 0.f;
+        // Configuration.getCanonical: the least hash, ties by Arrays.compare, then by variant
+        int32_t least32 = min(min(hash[0], hash[1]), min(hash[2], hash[3]));
+        least32 = __reduce_min_sync(kFull, least32);
+        int bestV = -1;
+        for (int from = 0;;) {
+            // the first variant >= from with the least hash
+            int v = INT32_MAX;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const int u = lane + 32 * g;
+                if (u < 2 * n && hash[g] == least32) {
+                    const int mine = u >= n ? 2 * (u - n) + 1 : 2 * u;
+                    if (mine >= from) v = min(v, mine);
+                }
+            }
+            v = __reduce_min_sync(kFull, v);
+            if (v == INT32_MAX) break;
+            float value[2];
+            build_row(S, hundredth, v, n, lane, value);
+            bool take = bestV < 0;
+            if (!take) {
+                const bool d0 = lane < n && value[0] != S.best[lane];
+                const bool d1 = lane + 32 < n && value[1] != S.best[lane + 32];
+                const unsigned b0 = __ballot_sync(kFull, d0), b1 = __ballot_sync(kFull, d1);
+                if (b0 | b1) {  // the least differing position decides
+                    const bool less = b0 ? value[0] < S.best[lane] : value[1] < S.best[lane + 32];
+                    take = __shfl_sync(kFull, (int)less, __ffs(b0 ? b0 : b1) - 1) != 0;
+                }
+                __syncwarp();
+            }
+            if (take) {
+                bestV = v;
+                S.best[lane] = value[0];
+                S.best[lane + 32] = value[1];
+            }
+            __syncwarp();
+            from = v + 1;
+        }
+        dst[lane] = S.best[lane];
+        dst[lane + 32] = S.best[lane + 32];
         if (lane == 0) {
-            A.hash[row] = bestHash;
+            A.hash[row] = least32;
             A.variant[row] = bestV;
         }
         __syncwarp();
@@ -288,7 +326,7 @@ int canonical_device(const uint8_t *spiDev, const uint8_t *nDev, int count, floa
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int blocks = (int)std::min<long long>(((long long)count + kWarps - 1) / kWarps, (long long)sms * 16);
+    const int blocks = (int)std::min<long long>(((long long)count + kWarps - 1) / kWarps, (long long)sms * 16 / kWarps * 4);
     CanonArgs A{spiDev, nDev, count, sigDev, hashDev, variantDev};
     canonical_kernel<<<blocks, kWarps * 32, 0, stream>>>(A);
     if (!ok(cudaGetLastError(), err, "canonical launch")) return -3;
