@@ -229,6 +229,30 @@ int tdp_mlp_adam(float *master, void *weight, const float *grad, float *m, float
                  float beta1, float beta2, float eps, int step, void *stream);
 int tdp_mlp_order(const float *scores, int ld, const uint8_t *n, int count, uint16_t *order, int order_stride,
                   void *stream);
+/* One training step of the model in one call (the products above, their gradients from untransposed
+ * operands, one Adam launch): x [rows x 1088] bf16, n and target per row (rows a multiple of 8);
+ * weights [out x in] bf16 with fp32 masters (the last layer padded to 5120 rows, the padding kept
+ * zero), biases and Adam moments (four weights, then four biases) fp32; all 16-byte aligned.
+ * step counts from 1.  workspace: tdp_mlp_train_workspace(rows) bytes, its contents are
+ * scratch.  means receives the mean loss and the top-1 accuracy before the step. */
+typedef struct tdp_mlp_train {
+    const void *x;
+    const uint8_t *n;
+    const int32_t *target;
+    int32_t rows;
+    int32_t step;
+    float *master[4];
+    void *weight[4];
+    float *bias[4];
+    float *m[8];
+    float *v[8];
+    float lr, beta1, beta2, eps;
+    void *workspace;
+    int64_t workspace_bytes;
+    float *means;
+} tdp_mlp_train;
+int64_t tdp_mlp_train_workspace(int rows);
+int tdp_mlp_train_step(const tdp_mlp_train *args, void *stream);
 /* 0 when no tensor-core wait has timed out since the last call (the flag is then cleared). */
 int tdp_mlp_error(void);
 

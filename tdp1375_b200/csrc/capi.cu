@@ -332,6 +332,49 @@ int tdp_mlp_adam(float *master, void *weight, const float *grad, float *m, float
     return launch_status("tdp_mlp_adam");
 }
 
+int64_t tdp_mlp_train_workspace(int rows) { return rows > 0 ? (int64_t)tdp::mlp::train_workspace(rows) : 0; }
+
+int tdp_mlp_train_step(const tdp_mlp_train *args, void *stream) {
+    if (!args || args->rows <= 0 || args->step < 1 || !args->x || !args->n || !args->target || !args->workspace ||
+        !args->means)
+        return fail(TDP_ERR_ARGUMENT, "tdp_mlp_train_step: bad arguments");
+    int *flag = mlp_error_flag();
+    if (!flag) return fail(TDP_ERR_OUT_OF_MEMORY, "tdp_mlp_train_step: error flag allocation failed");
+    tdp::mlp::TrainStep T{};
+    T.x = static_cast<const __nv_bfloat16 *>(args->x);
+    T.n = args->n;
+    T.target = args->target;
+    T.rows = args->rows;
+    T.step = args->step;
+    for (int l = 0; l < 8; ++l) {
+        if (l < 4) {
+            T.master[l] = args->master[l];
+            T.weight[l] = static_cast<__nv_bfloat16 *>(args->weight[l]);
+            T.bias[l] = args->bias[l];
+        }
+        T.m[l] = args->m[l];
+        T.v[l] = args->v[l];
+        const void *used[5] = {T.master[l & 3], T.weight[l & 3], T.bias[l & 3], T.m[l], T.v[l]};
+        for (const void *q : used)
+            if (l >= 4 && (!q || (reinterpret_cast<uintptr_t>(q) & 15u) != 0))
+                return fail(TDP_ERR_ARGUMENT, "tdp_mlp_train_step: parameters must be 16-byte aligned");
+        for (const void *q : {static_cast<const void *>(T.m[l]), static_cast<const void *>(T.v[l])})
+            if (!q || (reinterpret_cast<uintptr_t>(q) & 15u) != 0)
+                return fail(TDP_ERR_ARGUMENT, "tdp_mlp_train_step: parameters must be 16-byte aligned");
+    }
+    T.lr = args->lr;
+    T.beta1 = args->beta1;
+    T.beta2 = args->beta2;
+    T.eps = args->eps;
+    T.workspace = args->workspace;
+    T.workspaceBytes = (size_t)args->workspace_bytes;
+    T.means = args->means;
+    std::string err;
+    const int rc = tdp::mlp::train_step(T, flag, static_cast<cudaStream_t>(stream), err);
+    if (rc != 0) return fail(rc == -1 ? TDP_ERR_ARGUMENT : TDP_ERR_CUDA, err);
+    return 0;
+}
+
 int tdp_mlp_order(const float *scores, int ld, const uint8_t *n, int count, uint16_t *order, int order_stride,
                   void *stream) {
     tdp::mlp::order_by_score(scores, ld, n, 1, count, order, order_stride, static_cast<cudaStream_t>(stream));

@@ -3,7 +3,9 @@
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <cmath>
 #include <cstdint>
+#include <string>
 
 #include "mlp.h"
 #include "tdp_math.cuh"
@@ -67,70 +69,119 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-__global__ void softmax_xent_kernel(const float *logits, int ld, const uint8_t *nArr, const int32_t *target, int rows,
-                                    __nv_bfloat16 *dlogits, float *loss) {
+// The largest position k of every triple (i < j < k) of 32, in lexicographic order: column c of
+// the logits is valid for a state of n symbols when kLast[c] < n.
+struct LastTable {
+    alignas(4) uint8_t k[kTriples];
+    constexpr LastTable() : k() {
+        int c = 0;
+        for (int i = 0; i < 30; ++i)
+            for (int j = i + 1; j < 31; ++j)
+                for (int l = j + 1; l < 32; ++l) k[c++] = (uint8_t)l;
+    }
+};
+__device__ const LastTable kLast = LastTable();
+
+// One block of 128 threads per row; a thread owns the column pairs 2 threadIdx.x + 256 t and
+// keeps them in registers, so the row is read once and each exponential is taken once.  The sum
+// is that of 256 strided columns' sums, added within groups of 32 and then across the eight
+// groups, in one fixed order.  Bound: the row's bytes (20 KB in, 10 KB out) and the divisions;
+// the largest position of a column comes from a table (the decode of c into (i, j, k) in all
+// three passes over the row was the whole cost before).  4,096 rows on one B200: 255 us with
+// the decodes, 61 us with the table and one column per thread, 56 us in pairs.  top1 (or
+// null) receives 1 where the row's greatest logit, over all triples, is the target's.
+constexpr int kXentThreads = 128;
+constexpr int kXentPer = kTriplesPadded / 256;  // column pairs per thread
+static_assert(kTriples % 2 == 0 && kTriplesPadded % 256 == 0, "column pairs");
+
+template <bool kTop1>
+__global__ void __launch_bounds__(kXentThreads, 6) softmax_xent_kernel(const float *logits, int ld, const uint8_t *nArr,
+                                                                    const int32_t *target, int rows,
+                                                                    __nv_bfloat16 *dlogits, float *loss, float *top1) {
     const int r = blockIdx.x;
     if (r >= rows) return;
     const int n = nArr[r];
-    __shared__ float red[32];
+    __shared__ float red[8];
     const float *row = logits + (size_t)r * ld;
-    // column c = lex32(i,j,k) is valid when k < n; validity via a per-column decode is
-    // costly, so decode once per column with the inverse walk below.
+    const bool paired = ld % 2 == 0 && (reinterpret_cast<uintptr_t>(logits) & 7u) == 0 &&
+                        (reinterpret_cast<uintptr_t>(dlogits) & 3u) == 0;
+    float2 x[kXentPer];
+    unsigned long long valid = 0ull;  // bits 2t, 2t + 1: the pair's columns
     float mx = -FLT_MAX;
-    for (int c = threadIdx.x; c < kTriples; c += blockDim.x) {
-        // decode c -> (i,j,k) by counting
-        int rem = c, i = 0;
-        while (i < 29 && rem >= (31 - i) * (30 - i) / 2) rem -= (31 - i) * (30 - i) / 2, ++i;
-        int j = i + 1;
-        while (j < 30 && rem >= 31 - j) rem -= 31 - j, ++j;
-        const int k = j + 1 + rem;
-        if (k < n) mx = fmaxf(mx, row[c]);
+#pragma unroll
+    for (int t = 0; t < kXentPer; ++t) {
+        const int c = 2 * (int)threadIdx.x + 256 * t;
+        x[t] = make_float2(0.f, 0.f);
+        if (c < kTriples) {
+            if (paired) x[t] = *reinterpret_cast<const float2 *>(row + c);
+            else x[t] = make_float2(row[c], row[c + 1]);
+            const uint32_t last = *reinterpret_cast<const uint16_t *>(kLast.k + c);
+            if ((int)(last & 0xFFu) < n) valid |= 1ull << (2 * t), mx = fmaxf(mx, x[t].x);
+            if ((int)(last >> 8) < n) valid |= 2ull << (2 * t), mx = fmaxf(mx, x[t].y);
+        }
+    }
+    const int tgt = target[r];
+    bool beaten = false;  // some logit ranks before the target's (greater, or equal and earlier)
+    if (kTop1) {
+        const float tv = row[tgt];
+        const bool isNan = tv != tv;  // a NaN ranks as the greatest
+#pragma unroll
+        for (int t = 0; t < kXentPer; ++t) {
+            const int c = 2 * (int)threadIdx.x + 256 * t;
+            if (c < kTriples) {
+                if (!isNan) {
+                    beaten |= !(x[t].x <= tv) || (x[t].x == tv && c < tgt);
+                    beaten |= !(x[t].y <= tv) || (x[t].y == tv && c + 1 < tgt);
+                } else {
+                    beaten |= (x[t].x != x[t].x && c < tgt) || (x[t].y != x[t].y && c + 1 < tgt);
+                }
+            }
+        }
     }
     mx = warp_max(mx);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        float v = threadIdx.x < blockDim.x / 32 ? red[threadIdx.x] : -FLT_MAX;
-        v = warp_max(v);
-        if (threadIdx.x == 0) red[0] = v;
+    mx = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+    beaten = __syncthreads_or(beaten);
+    float2 part = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < kXentPer; ++t) {
+        x[t].x = __expf(x[t].x - mx);
+        x[t].y = __expf(x[t].y - mx);
+        if ((valid >> (2 * t)) & 1ull) part.x += x[t].x;
+        if ((valid >> (2 * t)) & 2ull) part.y += x[t].y;
     }
-    __syncthreads();
-    mx = red[0];
-    __syncthreads();
-    float sum = 0.f;
-    for (int c = threadIdx.x; c < kTriples; c += blockDim.x) {
-        int rem = c, i = 0;
-        while (i < 29 && rem >= (31 - i) * (30 - i) / 2) rem -= (31 - i) * (30 - i) / 2, ++i;
-        int j = i + 1;
-        while (j < 30 && rem >= 31 - j) rem -= 31 - j, ++j;
-        const int k = j + 1 + rem;
-        if (k < n) sum += __expf(row[c] - mx);
+    // a group of 32 columns is 16 lanes of pairs; its halving tree ends inside the pair
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+        part.x += __shfl_xor_sync(0xFFFFFFFFu, part.x, o);
+        part.y += __shfl_xor_sync(0xFFFFFFFFu, part.y, o);
     }
-    sum = warp_sum(sum);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+    if ((threadIdx.x & 15) == 0) red[threadIdx.x >> 4] = part.x + part.y;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        float v = threadIdx.x < blockDim.x / 32 ? red[threadIdx.x] : 0.f;
-        v = warp_sum(v);
-        if (threadIdx.x == 0) red[0] = v;
-    }
-    __syncthreads();
-    sum = red[0];
-    const int tgt = target[r];
+    // the eight groups' sums, halved as eight lanes of a warp would
+    const float sum = ((red[0] + red[4]) + (red[2] + red[6])) + ((red[1] + red[5]) + (red[3] + red[7]));
     const float inv = 1.f / (float)rows;
-    for (int c = threadIdx.x; c < ld; c += blockDim.x) {
-        float g = 0.f;
-        if (c < kTriples) {
-            int rem = c, i = 0;
-            while (i < 29 && rem >= (31 - i) * (30 - i) / 2) rem -= (31 - i) * (30 - i) / 2, ++i;
-            int j = i + 1;
-            while (j < 30 && rem >= 31 - j) rem -= 31 - j, ++j;
-            const int k = j + 1 + rem;
-            if (k < n) g = __expf(row[c] - mx) / sum - (c == tgt ? 1.f : 0.f);
+#pragma unroll
+    for (int t = 0; t < kXentPer; ++t) {
+        const int c = 2 * (int)threadIdx.x + 256 * t;
+        float2 g = make_float2(0.f, 0.f);
+        if ((valid >> (2 * t)) & 1ull) g.x = x[t].x / sum - (c == tgt ? 1.f : 0.f);
+        if ((valid >> (2 * t)) & 2ull) g.y = x[t].y / sum - (c + 1 == tgt ? 1.f : 0.f);
+        __nv_bfloat16 *const dst = dlogits + (size_t)r * ld + c;
+        if (paired && c + 1 < ld) {
+            *reinterpret_cast<__nv_bfloat162 *>(dst) = __floats2bfloat162_rn(g.x * inv, g.y * inv);
+        } else {
+            if (c < ld) dst[0] = __float2bfloat16_rn(g.x * inv);
+            if (c + 1 < ld) dst[1] = __float2bfloat16_rn(g.y * inv);
         }
-        dlogits[(size_t)r * ld + c] = __float2bfloat16_rn(g * inv);
     }
-    if (threadIdx.x == 0) loss[r] = -(row[tgt] - mx - __logf(sum));
+    for (int c = (int)threadIdx.x + kTriplesPadded; c < ld; c += kXentThreads)
+        dlogits[(size_t)r * ld + c] = __float2bfloat16_rn(0.f);
+    if (threadIdx.x == 0) {
+        loss[r] = -(row[tgt] - mx - __logf(sum));
+        if (kTop1) top1[r] = beaten ? 0.f : 1.f;
+    }
 }
 
 __global__ void transpose_kernel(const __nv_bfloat16 *in, int rows, int cols, __nv_bfloat16 *out) {
@@ -152,12 +203,56 @@ __global__ void relu_backward_kernel(__nv_bfloat16 *grad, const __nv_bfloat16 *a
         if (__bfloat162float(act[i]) <= 0.f) grad[i] = __float2bfloat16_rn(0.f);
 }
 
-__global__ void column_sums_kernel(const __nv_bfloat16 *grad, int rows, int cols, float *out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
+// 32 columns per block, 32 rows at a time, then a reduction over the rows' warps.
+__global__ void __launch_bounds__(1024) column_sums_kernel(const __nv_bfloat16 *grad, int rows, int cols, float *out) {
+    __shared__ float part[32][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int c = blockIdx.x * 32 + x;
     float s = 0.f;
-    for (int r = 0; r < rows; ++r) s += __bfloat162float(grad[(size_t)r * cols + c]);
-    out[c] = s;
+    if (c < cols)
+        for (int r = y; r < rows; r += 32) s += __bfloat162float(grad[(size_t)r * cols + c]);
+    part[y][x] = s;
+    __syncthreads();
+    const float v = warp_sum(part[x][y]);
+    if (x == 0 && blockIdx.x * 32 + y < cols) out[blockIdx.x * 32 + y] = v;
+}
+
+// Bias gradients of one training step, all layers in one launch: partial column sums over spans
+// of kSumRows rows.  A block takes 256 columns (32 threads of 8) and 8 rows at a time.
+constexpr int kSumRows = 64;
+
+struct ColumnSumArgs {
+    const __nv_bfloat16 *grad[4];
+    float *partials[4];  // [spans x cols]
+    int cols[4], firstBlock[4];
+    int rows;
+};
+
+__global__ void __launch_bounds__(256) column_partials_kernel(const __grid_constant__ ColumnSumArgs A) {
+    __shared__ float part[8][256 + 8];
+    int layer = 3;
+    while (layer > 0 && (int)blockIdx.x < A.firstBlock[layer]) --layer;
+    const int cols = A.cols[layer], x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int c = ((int)blockIdx.x - A.firstBlock[layer]) * 256 + x * 8;
+    float s[8] = {};
+    const int last = min((int)(blockIdx.y + 1) * kSumRows, A.rows);
+#pragma unroll 4
+    for (int r = (int)blockIdx.y * kSumRows + y; r < last; r += 8) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(A.grad[layer] + (size_t)r * cols + c));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            s[2 * j] += __uint_as_float(w[j] << 16);
+            s[2 * j + 1] += __uint_as_float(w[j] & 0xFFFF0000u);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part[y][x * 8 + j] = s[j];
+    __syncthreads();
+    float sum = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) sum += part[q][threadIdx.x];
+    A.partials[layer][(size_t)blockIdx.y * cols + ((int)blockIdx.x - A.firstBlock[layer]) * 256 + threadIdx.x] = sum;
 }
 
 __global__ void adam_kernel(float *master, __nv_bfloat16 *weight, const float *grad, float *m, float *v, size_t count,
@@ -171,6 +266,74 @@ __global__ void adam_kernel(float *master, __nv_bfloat16 *weight, const float *g
         const float w = master[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
         master[i] = w;
         weight[i] = __float2bfloat16_rn(w);
+    }
+}
+
+// One Adam step of all weights and biases in one launch, four elements per thread.  The gradient
+// is the sum of its partial products (spans of rows), added here so it never makes a pass of
+// its own.  Block 0 reduces the rows' losses and top-1 hits to their means; the biases, whose
+// sums have the most parts, come next, so the long chains start first.
+struct AdamSegment {
+    float *master;
+    __nv_bfloat16 *weight;  // null for a bias
+    const float *partials;  // [splits x count]
+    float *m, *v;
+    int splits, count, zeroFrom, firstBlock;  // elements from zeroFrom on are padding: weight 0
+};
+struct AdamArgs {
+    AdamSegment seg[8];
+    float lr, b1, b2, eps, c1, c2;
+    const float *loss, *top1;
+    float *means;
+    int rows;
+};
+constexpr int kAdamPerBlock = 1024;
+
+__global__ void __launch_bounds__(256) adam_step_kernel(const __grid_constant__ AdamArgs A) {
+    if (blockIdx.x == 0) {
+        __shared__ float sums[2][8];
+        float l = 0.f, h = 0.f;
+        for (int r = threadIdx.x; r < A.rows; r += 256) l += A.loss[r], h += A.top1[r];
+        l = warp_sum(l);
+        h = warp_sum(h);
+        if ((threadIdx.x & 31) == 0) sums[0][threadIdx.x >> 5] = l, sums[1][threadIdx.x >> 5] = h;
+        __syncthreads();
+        if (threadIdx.x < 2) {
+            float s = 0.f;
+            for (int w = 0; w < 8; ++w) s += sums[threadIdx.x][w];
+            A.means[threadIdx.x] = s / (float)A.rows;
+        }
+        return;
+    }
+    int k = 7;
+    while (k > 0 && (int)blockIdx.x < A.seg[k].firstBlock) --k;
+    const AdamSegment &S = A.seg[k];
+    const int i = ((int)blockIdx.x - S.firstBlock) * kAdamPerBlock + (int)threadIdx.x * 4;
+    if (i >= S.count) return;
+    float4 g = *reinterpret_cast<const float4 *>(S.partials + i);
+#pragma unroll 8
+    for (int q = 1; q < S.splits; ++q) {
+        const float4 t = *reinterpret_cast<const float4 *>(S.partials + (size_t)q * S.count + i);
+        g.x += t.x, g.y += t.y, g.z += t.z, g.w += t.w;
+    }
+    float4 m = *reinterpret_cast<const float4 *>(S.m + i), v = *reinterpret_cast<const float4 *>(S.v + i);
+    float4 w = *reinterpret_cast<const float4 *>(S.master + i);
+    auto step = [&](float gj, float &mj, float &vj, float &wj, int at) {
+        mj = A.b1 * mj + (1.f - A.b1) * gj;
+        vj = A.b2 * vj + (1.f - A.b2) * gj * gj;
+        wj = at < S.zeroFrom ? wj - A.lr * (mj / A.c1) / (sqrtf(vj / A.c2) + A.eps) : 0.f;
+    };
+    step(g.x, m.x, v.x, w.x, i);
+    step(g.y, m.y, v.y, w.y, i + 1);
+    step(g.z, m.z, v.z, w.z, i + 2);
+    step(g.w, m.w, v.w, w.w, i + 3);
+    *reinterpret_cast<float4 *>(S.m + i) = m;
+    *reinterpret_cast<float4 *>(S.v + i) = v;
+    *reinterpret_cast<float4 *>(S.master + i) = w;
+    if (S.weight) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(w.x, w.y), hi = __floats2bfloat162_rn(w.z, w.w);
+        *reinterpret_cast<uint2 *>(S.weight + i) =
+            make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
     }
 }
 
@@ -343,7 +506,8 @@ void build_features(const uint8_t *spi, const uint8_t *pi, const uint8_t *n, int
 
 void softmax_xent(const float *logits, int ld, const uint8_t *n, const int32_t *target, int rows,
                   __nv_bfloat16 *dlogits, float *loss, cudaStream_t stream) {
-    if (rows > 0) softmax_xent_kernel<<<rows, 256, 0, stream>>>(logits, ld, n, target, rows, dlogits, loss);
+    if (rows > 0)
+        softmax_xent_kernel<false><<<rows, kXentThreads, 0, stream>>>(logits, ld, n, target, rows, dlogits, loss, nullptr);
 }
 
 void transpose_bf16(const __nv_bfloat16 *in, int rows, int cols, __nv_bfloat16 *out, cudaStream_t stream) {
@@ -356,7 +520,7 @@ void relu_backward(__nv_bfloat16 *grad, const __nv_bfloat16 *act, size_t count, 
 }
 
 void column_sums(const __nv_bfloat16 *grad, int rows, int cols, float *out, cudaStream_t stream) {
-    column_sums_kernel<<<(cols + 255) / 256, 256, 0, stream>>>(grad, rows, cols, out);
+    column_sums_kernel<<<(cols + 31) / 32, 1024, 0, stream>>>(grad, rows, cols, out);
 }
 
 void adam_step(float *master, __nv_bfloat16 *weight, const float *grad, float *m, float *v, size_t count, float lr,
@@ -381,6 +545,125 @@ void level1_states(const uint8_t *spi, const uint8_t *pi, const uint8_t *n, int 
 void top_k(const float *scores, int ld, const uint8_t *n, int nStride, int count, int k, uint16_t *out, int outStride,
            cudaStream_t stream) {
     if (count > 0 && k > 0) topk_kernel<<<count, 256, 0, stream>>>(scores, ld, n, nStride, count, k, out, outStride);
+}
+
+// ---------------------------------------------------------------- one training step
+namespace {
+
+constexpr int kLayers = 4;
+constexpr int kOut[kLayers] = {kHidden, kHidden, kHidden, kTriplesPadded};
+constexpr int kIn[kLayers] = {kFeatures, kHidden, kHidden, kHidden};
+
+// Scratch of a step, carved from one caller-owned buffer in 256-byte pieces.
+struct TrainScratch {
+    __nv_bfloat16 *act[kLayers];   // act[l]: input of layer l (act[0] unused: x)
+    __nv_bfloat16 *grad[kLayers];  // grad[l]: gradient of layer l's output
+    float *logits, *loss, *top1;
+    float *weightParts[kLayers], *biasParts[kLayers];
+    size_t bytes;
+};
+
+TrainScratch carve(uint8_t *base, int rows) {
+    TrainScratch S{};
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        uint8_t *p = base + at;
+        at += (bytes + 255) & ~(size_t)255;
+        return static_cast<void *>(p);
+    };
+    const size_t R = (size_t)rows;
+    const int spans = (rows + kSumRows - 1) / kSumRows;
+    for (int l = 1; l < kLayers; ++l) S.act[l] = static_cast<__nv_bfloat16 *>(take(R * kHidden * 2));
+    S.logits = static_cast<float *>(take(R * kTriplesPadded * 4));
+    for (int l = 0; l < kLayers; ++l) {
+        S.grad[l] = static_cast<__nv_bfloat16 *>(take(R * kOut[l] * 2));
+        S.weightParts[l] =
+            static_cast<float *>(take((size_t)weight_grad_splits(rows, kOut[l], kIn[l]) * kOut[l] * kIn[l] * 4));
+        S.biasParts[l] = static_cast<float *>(take((size_t)spans * kOut[l] * 4));
+    }
+    S.loss = static_cast<float *>(take(R * 4));
+    S.top1 = static_cast<float *>(take(R * 4));
+    S.bytes = at;
+    return S;
+}
+
+}  // namespace
+
+size_t train_workspace(int rows) { return carve(nullptr, rows).bytes; }
+
+int train_step(const TrainStep &T, int *errorFlag, cudaStream_t stream, std::string &err) {
+    const int rows = T.rows;
+    if (rows % 8 != 0) {
+        err = "gemm operand must be 16-byte aligned with a row length that is a multiple of 8";
+        return -1;
+    }
+    const TrainScratch S = carve(static_cast<uint8_t *>(T.workspace), rows);
+    if (T.workspaceBytes < S.bytes) {
+        err = "tdp_mlp_train_step: workspace too small";
+        return -1;
+    }
+    const __nv_bfloat16 *act[kLayers] = {T.x, S.act[1], S.act[2], S.act[3]};
+    for (int l = 0; l < kLayers; ++l) {
+        void *out = l < 3 ? static_cast<void *>(S.act[l + 1]) : static_cast<void *>(S.logits);
+        const int rc = gemm_bf16(act[l], T.weight[l], rows, kOut[l], kIn[l], T.bias[l], l < 3, out, l == 3, kOut[l],
+                                 errorFlag, stream, err);
+        if (rc != 0) return rc;
+    }
+    softmax_xent_kernel<true><<<rows, kXentThreads, 0, stream>>>(S.logits, kTriplesPadded, T.n, T.target, rows, S.grad[3],
+                                                        S.loss, S.top1);
+    for (int l = kLayers - 1; l >= 0; --l) {
+        int rc = gemm_weight_grad(S.grad[l], act[l], rows, kOut[l], kIn[l], S.weightParts[l], errorFlag, stream, err);
+        if (rc == 0 && l > 0)
+            rc = gemm_input_grad(S.grad[l], T.weight[l], rows, kOut[l], kIn[l], act[l], S.grad[l - 1], errorFlag,
+                                 stream, err);
+        if (rc != 0) return rc;
+    }
+    const int spans = (rows + kSumRows - 1) / kSumRows;
+    ColumnSumArgs C{};
+    C.rows = rows;
+    int blocks = 0;
+    for (int l = 0; l < kLayers; ++l) {
+        C.grad[l] = S.grad[l];
+        C.partials[l] = S.biasParts[l];
+        C.cols[l] = kOut[l];
+        C.firstBlock[l] = blocks;
+        blocks += kOut[l] / 256;
+    }
+    column_partials_kernel<<<dim3(blocks, spans), 256, 0, stream>>>(C);
+    AdamArgs A{};
+    A.lr = T.lr;
+    A.b1 = T.beta1;
+    A.b2 = T.beta2;
+    A.eps = T.eps;
+    A.c1 = 1.f - powf(T.beta1, (float)T.step);
+    A.c2 = 1.f - powf(T.beta2, (float)T.step);
+    A.loss = S.loss;
+    A.top1 = S.top1;
+    A.means = T.means;
+    A.rows = rows;
+    blocks = 1;
+    for (int at = 0; at < 2 * kLayers; ++at) {
+        const int k = (at + kLayers) % (2 * kLayers), l = k % kLayers;
+        const bool bias = k >= kLayers;
+        AdamSegment &G = A.seg[at];
+        G.master = bias ? T.bias[l] : T.master[l];
+        G.weight = bias ? nullptr : T.weight[l];
+        G.partials = bias ? S.biasParts[l] : S.weightParts[l];
+        G.m = T.m[k];
+        G.v = T.v[k];
+        G.splits = bias ? spans : weight_grad_splits(rows, kOut[l], kIn[l]);
+        G.count = bias ? kOut[l] : kOut[l] * kIn[l];
+        G.zeroFrom = !bias && l == 3 ? kTriples * kHidden : G.count;
+        G.firstBlock = blocks;
+        blocks += (G.count + kAdamPerBlock - 1) / kAdamPerBlock;
+    }
+    adam_step_kernel<<<blocks, 256, 0, stream>>>(A);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        err = std::string("tdp_mlp_train_step: ") + cudaGetErrorString(e);
+        return -3;
+    }
+    return 0;
 }
 
 }  // namespace mlp

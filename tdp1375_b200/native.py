@@ -44,6 +44,14 @@ class EngineConfig(ctypes.Structure):
                 ("commute", ctypes.c_int32), ("probe_leaves", ctypes.c_int32)]
 
 
+class MlpTrain(ctypes.Structure):
+    _fields_ = [("x", ctypes.c_void_p), ("n", ctypes.c_void_p), ("target", ctypes.c_void_p), ("rows", ctypes.c_int32),
+                ("step", ctypes.c_int32), ("master", ctypes.c_void_p * 4), ("weight", ctypes.c_void_p * 4),
+                ("bias", ctypes.c_void_p * 4), ("m", ctypes.c_void_p * 8), ("v", ctypes.c_void_p * 8),
+                ("lr", ctypes.c_float), ("beta1", ctypes.c_float), ("beta2", ctypes.c_float), ("eps", ctypes.c_float),
+                ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_int64), ("means", ctypes.c_void_p)]
+
+
 assert ctypes.sizeof(Instance) == 136 and ctypes.sizeof(Result) == 208
 
 u8p = ctypes.POINTER(ctypes.c_uint8)
@@ -81,6 +89,8 @@ SIGNATURES = {
     "tdp_mlp_adam": (ctypes.c_int, [vp, vp, vp, vp, vp, ctypes.c_int64, ctypes.c_float, ctypes.c_float,
                                     ctypes.c_float, ctypes.c_float, ctypes.c_int, vp]),
     "tdp_mlp_order": (ctypes.c_int, [vp, ctypes.c_int, vp, ctypes.c_int, vp, ctypes.c_int, vp]),
+    "tdp_mlp_train_workspace": (ctypes.c_int64, [ctypes.c_int]),
+    "tdp_mlp_train_step": (ctypes.c_int, [ctypes.POINTER(MlpTrain), vp]),
     "tdp_mlp_error": (ctypes.c_int, []),
     "tdp_set_order_model": (ctypes.c_int, [ctypes.c_int] + [vp] * 8),
     "tdp_enable_order_model": (ctypes.c_int, [ctypes.c_int, ctypes.c_int]),

@@ -117,50 +117,21 @@ class OrderModel:
     def train_step(self, x, n, target, lr=1e-3):
         """One Adam step on a batch; returns (mean loss, top-1 accuracy)."""
         import torch
-        L = lib()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
         rows = x.shape[0]
-        logits, acts = self.forward(x)
-        dlogits = torch.empty(rows, TRIPLES_PADDED, device=x.device, dtype=torch.bfloat16)
-        loss = torch.empty(rows, device=x.device)
-        _check(L.tdp_mlp_softmax_xent(_ptr(logits), TRIPLES_PADDED, _ptr(n), _ptr(target), rows, _ptr(dlogits),
-                                      _ptr(loss), stream))
-        top1 = (logits[:, :TRIPLES].argmax(dim=1) == target.long()).float().mean()
-        grads_w, grads_b = [None] * 4, [None] * 4
-        grad = dlogits
-        for layer in (3, 2, 1, 0):
-            a = acts[layer]
-            out_dim, in_dim = LAYERS[layer]
-            # dW = grad^T @ a : A = grad^T [out x rows], B = a^T [in x rows]
-            gT = torch.empty(out_dim, rows, device=x.device, dtype=torch.bfloat16)
-            aT = torch.empty(in_dim, rows, device=x.device, dtype=torch.bfloat16)
-            _check(L.tdp_mlp_transpose(_ptr(grad), rows, out_dim, _ptr(gT), stream))
-            _check(L.tdp_mlp_transpose(_ptr(a), rows, in_dim, _ptr(aT), stream))
-            grads_w[layer] = gemm(gT, aT, out_fp32=True)
-            gb = torch.empty(out_dim, device=x.device)
-            _check(L.tdp_mlp_column_sums(_ptr(grad), rows, out_dim, _ptr(gb), stream))
-            grads_b[layer] = gb
-            if layer > 0:
-                # d(input) = grad @ W : B operand = W^T [in x out]
-                wT = torch.empty(in_dim, out_dim, device=x.device, dtype=torch.bfloat16)
-                _check(L.tdp_mlp_transpose(_ptr(self.weight[layer]), out_dim, in_dim, _ptr(wT), stream))
-                g_in = gemm(grad, wT)
-                _check(L.tdp_mlp_relu_backward(_ptr(g_in), _ptr(acts[layer]), g_in.numel(), stream))
-                grad = g_in
+        bytes_needed = int(lib().tdp_mlp_train_workspace(rows))
+        workspace = torch.empty(bytes_needed, dtype=torch.uint8, device=x.device)
+        means = torch.empty(2, device=x.device)
+        four, eight = ctypes.c_void_p * 4, ctypes.c_void_p * 8
+        args = native.MlpTrain(x.data_ptr(), n.data_ptr(), target.data_ptr(), rows, self.step + 1,
+                               four(*[t.data_ptr() for t in self.master]), four(*[t.data_ptr() for t in self.weight]),
+                               four(*[t.data_ptr() for t in self.bias]), eight(*[t.data_ptr() for t in self.m]),
+                               eight(*[t.data_ptr() for t in self.v]), lr, 0.9, 0.999, 1e-8, workspace.data_ptr(),
+                               bytes_needed, means.data_ptr())
+        _check(lib().tdp_mlp_train_step(ctypes.byref(args),
+                                        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
         self.step += 1
-        for layer in range(4):
-            _check(L.tdp_mlp_adam(_ptr(self.master[layer]), _ptr(self.weight[layer]), _ptr(grads_w[layer]),
-                                  _ptr(self.m[layer]), _ptr(self.v[layer]), self.master[layer].numel(),
-                                  ctypes.c_float(lr), ctypes.c_float(0.9), ctypes.c_float(0.999),
-                                  ctypes.c_float(1e-8), self.step, stream))
-            bias_bf = torch.empty_like(self.bias[layer], dtype=torch.bfloat16)
-            _check(L.tdp_mlp_adam(_ptr(self.bias[layer]), _ptr(bias_bf), _ptr(grads_b[layer]), _ptr(self.m[4 + layer]),
-                                  _ptr(self.v[4 + layer]), self.bias[layer].numel(), ctypes.c_float(lr),
-                                  ctypes.c_float(0.9), ctypes.c_float(0.999), ctypes.c_float(1e-8), self.step, stream))
-        with torch.no_grad():
-            self.master[3][TRIPLES:] = 0.0
-            self.weight[3][TRIPLES:] = 0.0
-        return float(loss.mean()), float(top1)
+        loss, top1 = means.tolist()
+        return loss, top1
 
     def install(self, slot: int, enable: bool = True, levels: int = 1) -> None:
         """Copies the weights into the search slot and turns ordering on: levels = 1 orders each
