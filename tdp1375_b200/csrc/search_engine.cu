@@ -90,6 +90,13 @@ SearchSlot::SearchSlot(int device, int64_t queueBytesBudget, int dedupTableSize)
     *hCancelValue_ = 1;
     check(cudaEventCreate(&evStart_), "cudaEventCreate");
     check(cudaEventCreate(&evStop_), "cudaEventCreate");
+    // the kernels' shared memory is above the 48 KB a launch may take unasked
+    check(cudaFuncSetAttribute(dev::search_engine_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(dev::kWarpsPerBlock * sizeof(dev::WarpShared<1>))),
+          "shared memory");
+    check(cudaFuncSetAttribute(dev::search_engine_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(dev::kWarpsPerBlock * sizeof(dev::WarpShared<2>))),
+          "shared memory");
     triples_ = device_triples(device);
     check(cudaDeviceGetAttribute(&numSMs_, cudaDevAttrMultiProcessorCount, device), "SM count");
 
@@ -322,13 +329,9 @@ void SearchSlot::launchClass(int cls, int offset, int count) {
 
     int blocksPerSM = 0;
     const int threads = dev::kWarpsPerBlock * 32;
-    if (cls == 0) {
-        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocksPerSM, dev::search_engine_kernel<1>, threads, 0),
-              "occupancy");
-    } else {
-        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocksPerSM, dev::search_engine_kernel<2>, threads, 0),
-              "occupancy");
-    }
+    auto *const kernel = cls == 0 ? dev::search_engine_kernel<1> : dev::search_engine_kernel<2>;
+    const size_t smem = dev::kWarpsPerBlock * (cls == 0 ? sizeof(dev::WarpShared<1>) : sizeof(dev::WarpShared<2>));
+    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocksPerSM, kernel, threads, smem), "occupancy");
     if (cfg_.blocks_per_sm > 0) blocksPerSM = std::min(blocksPerSM, cfg_.blocks_per_sm);
     blocksPerSM = std::max(1, blocksPerSM);
     // every warp of the grid needs a mailbox
@@ -336,11 +339,7 @@ void SearchSlot::launchClass(int cls, int offset, int count) {
     P.maxInFlight = cfg_.warps_per_instance > 0
                         ? std::max(1, grid * dev::kWarpsPerBlock / cfg_.warps_per_instance)
                         : 0;
-    if (cls == 0) {
-        dev::search_engine_kernel<1><<<grid, threads, 0, stream_>>>(P);
-    } else {
-        dev::search_engine_kernel<2><<<grid, threads, 0, stream_>>>(P);
-    }
+    kernel<<<grid, threads, smem, stream_>>>(P);
     check(cudaGetLastError(), "launch search_engine_kernel");
     check(cudaMemcpyAsync(hCtl_ + cls, dCtl_, sizeof(EngineCtl), cudaMemcpyDeviceToHost, stream_), "read ctl");
     launched_[cls] = true;

@@ -36,6 +36,8 @@
 // ends the launch with an error flag instead of hanging the GPU.
 #pragma once
 
+#include <type_traits>
+
 #include "engine.cuh"
 
 namespace tdp {
@@ -491,31 +493,42 @@ __device__ __forceinline__ void apply_move(const uint32_t (&w)[NW], uint32_t (&o
     }
 }
 
-// Restricted child enumerations (n <= 32, one position per lane).  Both rest on the cycle
-// structure of spi: a child's odd-cycle count changes by +2 only if its three symbols lie
-// in one cycle, or two lie in one even-length cycle and the third in another even-length
-// cycle; a triple over three distinct cycles changes the count by -2, or by 0 only when two
-// of those cycles have even length.
+// Restricted child enumerations.  Both rest on the cycle structure of spi: a child's odd-cycle
+// count changes by +2 only if its three symbols lie in one cycle, or two lie in one even-length
+// cycle and the third in another even-length cycle; a triple over three distinct cycles changes
+// the count by -2, or by 0 only when two of those cycles have even length.
 //
 // * Pairs (mode 1).  When no child with a -2 change is useful, and either 0-changes are
 //   useless too or the node has at most one even-length cycle, every useful child has two
 //   of its three symbols in one cycle.  The frame enumerates position pairs p < q whose
-//   symbols share a cycle, one pair per chunk, with the lane as the third position r; a
-//   triple lying in one cycle is taken only from its two smallest positions.
+//   symbols share a cycle, with the lanes as the third position r: NW chunks per pair, index
+//   NW * pair + (r / 32); a triple lying in one cycle is taken only from its two smallest
+//   positions.
 // * Triples (mode 2).  When only +2 children are useful and the node has at most one
 //   even-length cycle, every useful child takes its three symbols from one cycle.  The
 //   frame enumerates the position triples p < q < r inside each cycle, 32 per chunk, from
 //   a list the warp writes to shared memory at frame set-up (at most kMaxTriples entries;
 //   a larger frame uses pairs).  In searches at the ratio limit this is nearly every frame,
 //   and a frame then needs one or two chunks instead of one per same-cycle pair.
+//
+// With two words per lane (n > 32) a dense frame is C(n, 3) / 32 chunks, 223 at n = 36, where
+// its same-cycle triples are one: the staged calls of configurations of the combination step
+// (n = 24..42, a third of them above 32) took 26.6 ms per 8 configurations with dense frames
+// above 32 symbols and 20.9 ms with the restricted ones.
 constexpr int kMaxTriples = 256;
 
+// Positions of one lane: lane and, for NW = 2, lane + 32; position order is all of the first
+// word's lanes, then the second's.
+template <int NW>
+using PosMask = std::conditional_t<NW == 1, uint32_t, uint64_t>;
+
+template <int NW>
 struct SparseFrame {
-    uint32_t same;       // positions > lane whose symbol shares the cycle of pi[lane]
-    uint32_t incl;       // inclusive prefix over lanes of popc(same) (pairs) or C(popc(same), 2) (triples)
-    uint32_t leaderPos;  // cycle leader of pi[lane]
-    int np;              // number of pairs or triples
-    int mode;            // 0 dense, 1 pairs, 2 triples
+    PosMask<NW> same[NW];    // later positions whose symbol shares the cycle of this position's
+    uint32_t incl[NW];       // inclusive prefix over positions of |same| (pairs) or C(|same|, 2) (triples)
+    uint32_t leaderPos[NW];  // cycle leader of this position's symbol
+    int np;                  // number of pair chunks or triples
+    int mode;                // 0 dense, 1 pairs, 2 triples
 };
 
 struct PairSel {
@@ -523,113 +536,178 @@ struct PairSel {
     uint32_t leader;
 };
 
-// allow: 0 dense only, 1 pairs, 2 pairs and triples.  triList (or null) receives the
-// triple list of a triple-mode frame; pass null to classify a frame without touching the
-// list of the frame being enumerated.
+__device__ __forceinline__ int count_bits(uint32_t m) { return __popc(m); }
+__device__ __forceinline__ int count_bits(uint64_t m) { return __popcll(m); }
+__device__ __forceinline__ int first_bit(uint32_t m) { return __ffs(m) - 1; }
+__device__ __forceinline__ int first_bit(uint64_t m) { return __ffsll((long long)m) - 1; }
+
+// Inclusive prefix of v over all positions, in position order; returns the total.
 template <int NW>
-__device__ __forceinline__ SparseFrame sparse_setup(const uint32_t (&w)[NW], int n, int lane, int even,
-                                                    uint64_t satMask, uint64_t expMask, int allow,
-                                                    uint32_t *triList) {
-    SparseFrame sf;
-    sf.same = 0u;
-    sf.incl = 0u;
-    sf.leaderPos = 0u;
-    sf.np = 0;
-    sf.mode = 0;
-    if constexpr (NW != 1) {
-        return sf;
-    } else {
-        if (allow <= 0) return sf;
-        const uint64_t useful = satMask | expMask;
-        const bool neg = even >= 2 && ((useful >> (even - 2)) & 1ull);
-        if (neg) return sf;
-        const bool zero = (useful >> even) & 1ull;
-        const bool isLeader = lane < n && w_leader(w[0]) == (uint32_t)lane;
-        const int evenLen = __popc(__ballot_sync(kFull, isLeader && (w_len(w[0]) & 1u) == 0u));
-        if (zero && evenLen >= 2) return sf;
-        const uint32_t leaderPos = w_leader(gather<1>(w, w_pi(w[0])));
-        const uint32_t key = (lane < n) ? leaderPos : 64u + (uint32_t)lane;
-        const uint32_t same = __match_any_sync(kFull, key) & ~((2u << lane) - 1u);
-        sf.same = same;
-        sf.leaderPos = leaderPos;
-        const uint32_t k = (uint32_t)__popc(same);
-        if (allow >= 2 && !zero && evenLen <= 1) {
-            const uint32_t c2 = k * (k - 1u) / 2u;
-            uint32_t incl = c2;
+__device__ __forceinline__ int prefix_positions(const uint32_t (&v)[NW], uint32_t (&incl)[NW], int lane) {
+    uint32_t before = 0u;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(kFull, incl, o);
-                if (lane >= o) incl += y;
-            }
-            const int total = (int)__shfl_sync(kFull, incl, 31);
-            if (total <= kMaxTriples) {
-                if (triList) {
-                    __syncwarp();  // every lane is done reading the previous frame's list
-                    uint32_t at = incl - c2;
-                    uint32_t m1 = same;
-                    while (m1) {
-                        const uint32_t q = (uint32_t)(__ffs(m1) - 1);
-                        m1 &= m1 - 1u;
-                        uint32_t m2 = m1;
-                        while (m2) {
-                            const uint32_t r = (uint32_t)(__ffs(m2) - 1);
-                            m2 &= m2 - 1u;
-                            triList[at++] = pack_triple((uint32_t)lane, q, r);
-                        }
-                    }
-                    __syncwarp();
-                }
-                sf.incl = incl;
-                sf.np = total;
-                sf.mode = 2;
-                return sf;
-            }
-        }
-        uint32_t incl = k;
+    for (int h = 0; h < NW; ++h) {
+        uint32_t x = v[h];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += y;
+            const uint32_t y = __shfl_up_sync(kFull, x, o);
+            if (lane >= o) x += y;
         }
-        sf.incl = incl;
-        sf.np = (int)__shfl_sync(kFull, incl, 31);
-        sf.mode = 1;
-        return sf;
+        incl[h] = before + x;
+        before = __shfl_sync(kFull, incl[h], 31);
+    }
+    return (int)before;
+}
+
+// allow: 0 dense only, 1 pairs, 2 pairs and triples.  triList (or null) receives the
+// triple list of a triple-mode frame; pass null to classify a frame without touching the
+// list of the frame being enumerated.  cycles: scratch of the warp (NW = 2).
+template <int NW>
+__device__ __forceinline__ SparseFrame<NW> sparse_setup(const uint32_t (&w)[NW], int n, int lane, int even,
+                                                        uint64_t satMask, uint64_t expMask, int allow,
+                                                        uint32_t *triList, uint32_t *cycles) {
+    using Mask = PosMask<NW>;
+    SparseFrame<NW> sf;
+#pragma unroll
+    for (int h = 0; h < NW; ++h) {
+        sf.same[h] = 0u;
+        sf.incl[h] = 0u;
+        sf.leaderPos[h] = 0u;
+    }
+    sf.np = 0;
+    sf.mode = 0;
+    if (allow <= 0) return sf;
+    const uint64_t useful = satMask | expMask;
+    const bool neg = even >= 2 && ((useful >> (even - 2)) & 1ull);
+    if (neg) return sf;
+    const bool zero = (useful >> even) & 1ull;
+    int evenLen = 0;
+#pragma unroll
+    for (int h = 0; h < NW; ++h) {
+        const int x = lane + 32 * h;
+        const bool isLeader = x < n && w_leader(w[h]) == (uint32_t)x;
+        evenLen += __popc(__ballot_sync(kFull, isLeader && (w_len(w[h]) & 1u) == 0u));
+    }
+    if (zero && evenLen >= 2) return sf;
+    uint32_t k[NW];
+    if constexpr (NW == 1) {
+        const uint32_t leaderPos = w_leader(gather<1>(w, w_pi(w[0])));
+        const uint32_t key = (lane < n) ? leaderPos : 64u + (uint32_t)lane;
+        sf.same[0] = __match_any_sync(kFull, key) & ~((2u << lane) - 1u);
+        sf.leaderPos[0] = leaderPos;
+        k[0] = (uint32_t)__popc(sf.same[0]);
+    } else {
+        // position sets per cycle leader, in shared memory: 64 words for the low positions, then
+        // 64 for the high ones
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cycles[lane + 32 * q] = 0u;
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            sf.leaderPos[h] = w_leader(gather<NW>(w, w_pi(w[h])));
+            if (lane + 32 * h < n) atomicOr(&cycles[64 * h + sf.leaderPos[h]], 1u << lane);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int x = lane + 32 * h;
+            const uint64_t all = (uint64_t)cycles[sf.leaderPos[h]] | ((uint64_t)cycles[64 + sf.leaderPos[h]] << 32);
+            sf.same[h] = x < n ? all & ~((2ull << x) - 1ull) : 0ull;
+            k[h] = (uint32_t)__popcll(sf.same[h]);
+        }
+        __syncwarp();
+    }
+    if (allow >= 2 && !zero && evenLen <= 1) {
+        uint32_t c2[NW];
+#pragma unroll
+        for (int h = 0; h < NW; ++h) c2[h] = k[h] * (k[h] - 1u) / 2u;
+        const int total = prefix_positions<NW>(c2, sf.incl, lane);
+        if (total <= kMaxTriples) {
+            if (triList) {
+                __syncwarp();  // every lane is done reading the previous frame's list
+#pragma unroll
+                for (int h = 0; h < NW; ++h) {
+                    uint32_t at = sf.incl[h] - c2[h];
+                    Mask m1 = sf.same[h];
+                    while (m1) {
+                        const uint32_t q = (uint32_t)first_bit(m1);
+                        m1 &= m1 - 1u;
+                        Mask m2 = m1;
+                        while (m2) {
+                            const uint32_t r = (uint32_t)first_bit(m2);
+                            m2 &= m2 - 1u;
+                            triList[at++] = pack_triple((uint32_t)(lane + 32 * h), q, r);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            sf.np = total;
+            sf.mode = 2;
+            return sf;
+        }
+    }
+    sf.np = NW * prefix_positions<NW>(k, sf.incl, lane);
+    sf.mode = 1;
+    return sf;
+}
+
+// The position that owns prefix index u (uniform), its mask and the prefix before it.
+template <int NW>
+__device__ __forceinline__ int sparse_owner(const SparseFrame<NW> &sf, int u, PosMask<NW> &mask, uint32_t &incl) {
+    const unsigned owner = __ballot_sync(kFull, sf.incl[0] > (uint32_t)u);
+    if constexpr (NW == 1) {
+        const int p = __ffs(owner) - 1;
+        mask = __shfl_sync(kFull, sf.same[0], p);
+        incl = __shfl_sync(kFull, sf.incl[0], p);
+        return p;
+    } else {
+        const int h = owner ? 0 : 1;
+        const int l = __ffs(owner ? owner : __ballot_sync(kFull, sf.incl[1] > (uint32_t)u)) - 1;
+        mask = shfl64(h ? sf.same[1] : sf.same[0], l);
+        incl = __shfl_sync(kFull, h ? sf.incl[1] : sf.incl[0], l);
+        return l + 32 * h;
     }
 }
 
 // Decodes pair index u (uniform) into positions p < q.
-__device__ __forceinline__ PairSel sparse_pair(const SparseFrame &sf, int u) {
-    const unsigned owner = __ballot_sync(kFull, sf.incl > (uint32_t)u);
-    const int p = __ffs(owner) - 1;
-    const uint32_t sameP = __shfl_sync(kFull, sf.same, p);
-    const uint32_t exclP = __shfl_sync(kFull, sf.incl, p) - (uint32_t)__popc(sameP);
-    uint32_t m = sameP;
-    for (uint32_t t = (uint32_t)u - exclP; t > 0u; --t) m &= m - 1u;
+template <int NW>
+__device__ __forceinline__ PairSel sparse_pair(const SparseFrame<NW> &sf, int u) {
+    PosMask<NW> m;
+    uint32_t inclP;
     PairSel ps;
-    ps.p = p;
-    ps.q = __ffs(m) - 1;
-    ps.leader = __shfl_sync(kFull, sf.leaderPos, p);
+    ps.p = sparse_owner<NW>(sf, u, m, inclP);
+    for (uint32_t t = (uint32_t)u - (inclP - (uint32_t)count_bits(m)); t > 0u; --t) m &= m - 1u;
+    ps.q = first_bit(m);
+    ps.leader = gather<NW>(sf.leaderPos, (uint32_t)ps.p);
     return ps;
+}
+
+// The triple of pair p < q and third position r.
+__device__ __forceinline__ uint32_t pair_triple(const PairSel &ps, int r) {
+    return r < ps.p ? pack_triple((uint32_t)r, (uint32_t)ps.p, (uint32_t)ps.q)
+           : r < ps.q ? pack_triple((uint32_t)ps.p, (uint32_t)r, (uint32_t)ps.q)
+                      : pack_triple((uint32_t)ps.p, (uint32_t)ps.q, (uint32_t)r);
 }
 
 // Triple index u (uniform) of a triple-mode frame, decoded without its list, in list order:
 // owner position p, then the v-th pair q < r of the positions in same(p) (lexicographic).
-__device__ __forceinline__ uint32_t triple_at(const SparseFrame &sf, int u) {
-    const unsigned owner = __ballot_sync(kFull, sf.incl > (uint32_t)u);
-    const int p = __ffs(owner) - 1;
-    const uint32_t sameP = __shfl_sync(kFull, sf.same, p);
-    const uint32_t k = (uint32_t)__popc(sameP);
-    uint32_t v = (uint32_t)u - (__shfl_sync(kFull, sf.incl, p) - k * (k - 1u) / 2u);
-    uint32_t m1 = sameP, q = 0u, r = 0u;
-    for (uint32_t it = 0; it < 32u && m1; ++it) {
-        q = (uint32_t)(__ffs(m1) - 1);
+template <int NW>
+__device__ __forceinline__ uint32_t triple_at(const SparseFrame<NW> &sf, int u) {
+    PosMask<NW> m1;
+    uint32_t inclP;
+    const int p = sparse_owner<NW>(sf, u, m1, inclP);
+    const uint32_t k = (uint32_t)count_bits(m1);
+    uint32_t v = (uint32_t)u - (inclP - k * (k - 1u) / 2u);
+    uint32_t q = 0u, r = 0u;
+    for (uint32_t it = 0; it < 32u * NW && m1; ++it) {
+        q = (uint32_t)first_bit(m1);
         m1 &= m1 - 1u;
-        const uint32_t cnt = (uint32_t)__popc(m1);
+        const uint32_t cnt = (uint32_t)count_bits(m1);
         if (v < cnt) {
-            uint32_t m2 = m1;
+            PosMask<NW> m2 = m1;
             for (uint32_t t = v; t > 0u; --t) m2 &= m2 - 1u;
-            r = (uint32_t)(__ffs(m2) - 1);
+            r = (uint32_t)first_bit(m2);
             break;
         }
         v -= cnt;
@@ -651,7 +729,8 @@ template <int NW>
 struct WarpShared {
     uint32_t words[kMaxDepth + 1][NW * 32];
     FrameRec<KeyTraits<NW>::KW> frames[kMaxDepth + 1];
-    uint32_t tri[NW == 1 ? kMaxTriples : 1];  // triple list of the frame being enumerated
+    uint32_t tri[kMaxTriples];                   // triple list of the frame being enumerated
+    uint32_t cycles[NW == 1 ? 1 : 128];          // sparse_setup's scratch
     uint64_t rules[32];                       // success (0..15) and expansion (16..31) tables of the instance
     unsigned long long taskNodes, taskChildren;  // counters of the task in hand
     int rank1;                                   // root-order rank of the current first-level node (-1: none)
@@ -663,7 +742,8 @@ template <int NW>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_engine_kernel(const EngineParams P) {
     using K = KeyTraits<NW>;
     constexpr int KW = K::KW;
-    __shared__ WarpShared<NW> smem[kWarpsPerBlock];
+    extern __shared__ __align__(16) uint8_t smemRaw[];
+    WarpShared<NW> *const smem = reinterpret_cast<WarpShared<NW> *>(smemRaw);
     const int lane = (int)(threadIdx.x & 31u);
     WarpShared<NW> &S = smem[threadIdx.x >> 5];
     EngineCtl *ctl = P.ctl;
@@ -842,7 +922,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
             return __ldg(trip + t);
         };
         auto denseEnd = [&](int g) -> int { return T + (listOf(g) ? P.order2List : 0); };
-        SparseFrame sf = sparse_setup<NW>(w, n, lane, even, satMask, expMask, ordered(f) ? 0 : P.sparse, S.tri);
+        SparseFrame<NW> sf =
+            sparse_setup<NW>(w, n, lane, even, satMask, expMask, ordered(f) ? 0 : P.sparse, S.tri, S.cycles);
         // A donated range is in the units of its frame's mode (the receiver derives the same
         // mode from the same node); hi = 0xFFFF covers every child.
         if (hi == 0xFFFF) end = sf.mode ? sf.np : denseEnd(f);
@@ -875,7 +956,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                     for (int h = 0; h < NW; ++h) w[h] = S.words[f][h * 32 + lane];
                     satMask = S.rules[f + 1];
                     expMask = S.rules[16 + f + 1];
-                    sf = sparse_setup<NW>(w, n, lane, even, satMask, expMask, ordered(f) ? 0 : P.sparse, S.tri);
+                    sf = sparse_setup<NW>(w, n, lane, even, satMask, expMask, ordered(f) ? 0 : P.sparse, S.tri, S.cycles);
                     continue;
                 }
                 if (++poll >= P.pollInterval) {
@@ -956,16 +1037,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                                 for (int h = 0; h < NW; ++h) wg[h] = S.words[g][h * 32 + lane];
                                 const uint64_t gSat = S.rules[g + 1];
                                 const uint64_t gExp = S.rules[16 + g + 1];
-                                const SparseFrame gsf =
-                                    sparse_setup<NW>(wg, n, lane, gEven, gSat, gExp, ordered(g) ? 0 : P.sparse, nullptr);
+                                const SparseFrame<NW> gsf = sparse_setup<NW>(
+                                    wg, n, lane, gEven, gSat, gExp, ordered(g) ? 0 : P.sparse, nullptr, S.cycles);
                                 uint32_t ctr;
                                 if (gsf.mode == 1) {
-                                    const PairSel ps = sparse_pair(gsf, gChunk);
-                                    ctr = (l < ps.p) ? pack_triple(l, ps.p, ps.q)
-                                                     : (l < ps.q) ? pack_triple(ps.p, l, ps.q)
-                                                                  : pack_triple(ps.p, ps.q, l);
+                                    ctr = pair_triple(sparse_pair<NW>(gsf, gChunk / NW), l + 32 * (gChunk % NW));
                                 } else if (gsf.mode == 2) {
-                                    ctr = triple_at(gsf, gChunk + l);
+                                    ctr = triple_at<NW>(gsf, gChunk + l);
                                 } else {
                                     const int t = gChunk + l;
                                     ctr = decode(g, t);
@@ -1057,25 +1135,20 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                 int nValid;
                 chunk = cursor;
                 if (sf.mode == 1) {
-                    // one same-cycle position pair (p, q) per chunk, lane = third position r
+                    // one same-cycle position pair (p, q), the lanes as the third position r
                     cursor += 1;
-                    const PairSel ps = sparse_pair(sf, chunk);
-                    const uint32_t r = (uint32_t)lane;
-                    valid = (int)r < n && (int)r != ps.p && (int)r != ps.q &&
-                            (sf.leaderPos != ps.leader || (int)r > ps.q);
-                    const uint32_t symP = w_pi(__shfl_sync(kFull, w[0], ps.p));
-                    const uint32_t symQ = w_pi(__shfl_sync(kFull, w[0], ps.q));
-                    const uint32_t symR = w_pi(w[0]);
-                    if ((int)r < ps.p) {
-                        tr = pack_triple(r, ps.p, ps.q);
-                        a = symR, b = symP, c = symQ;
-                    } else if ((int)r < ps.q) {
-                        tr = pack_triple(ps.p, r, ps.q);
-                        a = symP, b = symR, c = symQ;
-                    } else {
-                        tr = pack_triple(ps.p, ps.q, r);
-                        a = symP, b = symQ, c = symR;
-                    }
+                    const PairSel ps = sparse_pair<NW>(sf, chunk / NW);
+                    const int half = chunk % NW;
+                    const int r = lane + 32 * half;
+                    const uint32_t leaderR = NW == 2 && half ? sf.leaderPos[NW - 1] : sf.leaderPos[0];
+                    valid = r < n && r != ps.p && r != ps.q && (leaderR != ps.leader || r > ps.q);
+                    const uint32_t symP = w_pi(gather<NW>(w, (uint32_t)ps.p));
+                    const uint32_t symQ = w_pi(gather<NW>(w, (uint32_t)ps.q));
+                    const uint32_t symR = w_pi(NW == 2 && half ? w[NW - 1] : w[0]);
+                    tr = pair_triple(ps, r);
+                    a = r < ps.p ? symR : symP;
+                    b = r < ps.p ? symP : r < ps.q ? symR : symQ;
+                    c = r < ps.q ? symQ : symR;
                     if (!valid) tr = a = b = c = 0u;
                     nValid = __popc(__ballot_sync(kFull, valid));
                 } else {
@@ -1177,10 +1250,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
             pending &= pending - 1u;
             uint32_t tr;
             if (sf.mode == 1) {
-                const PairSel ps = sparse_pair(sf, chunk);
-                const int r = l;
-                tr = (r < ps.p) ? pack_triple(r, ps.p, ps.q)
-                                : (r < ps.q) ? pack_triple(ps.p, r, ps.q) : pack_triple(ps.p, ps.q, r);
+                tr = pair_triple(sparse_pair<NW>(sf, chunk / NW), l + 32 * (chunk % NW));
             } else if (sf.mode == 2) {
                 tr = S.tri[chunk + l];
             } else {
@@ -1231,7 +1301,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
             for (int h = 0; h < NW; ++h) S.words[f][h * 32 + lane] = w[h];
             satMask = S.rules[f + 1];
             expMask = S.rules[16 + f + 1];
-            sf = sparse_setup<NW>(w, n, lane, even, satMask, expMask, ordered(f) ? 0 : P.sparse, S.tri);
+            sf = sparse_setup<NW>(w, n, lane, even, satMask, expMask, ordered(f) ? 0 : P.sparse, S.tri, S.cycles);
             cursor = 0;
             end = sf.mode ? sf.np : denseEnd(f);
             pending = 0u;
