@@ -10,6 +10,15 @@ pytestmark = pytest.mark.gpu
 R1375 = float(np.float32(2) / np.float32(1.375))
 
 
+@pytest.fixture(scope="module")
+def slots(native_lib):
+    """Slots of this module alone: other modules destroy and create theirs."""
+    from tdp1375_b200 import GPUSortingSearch
+    GPUSortingSearch(1, 2, 256 << 20, 1 << 21)
+    yield
+    GPUSortingSearch.destroySlots()
+
+
 def instance(rng, n, lengths, unoriented):
     """pi a random arrangement; cycles of the given lengths on random symbols, the rest fixed."""
     pi = rng.permutation(n)
@@ -33,7 +42,7 @@ SHAPES = [([3] * 11, 33, 3, False), ([3] * 12, 36, 3, False), ([5, 3, 3], 34, 6,
 
 
 @pytest.mark.parametrize("lengths,n,depth,full", SHAPES)
-def test_enumeration_modes_match_oracle(gpu_searcher, oracle, lengths, n, depth, full):
+def test_enumeration_modes_match_oracle(slots, oracle, lengths, n, depth, full):
     from tdp1375_b200 import api, make_instances, native, search_batch
     rng = np.random.Generator(np.random.PCG64([n, depth, len(lengths)]))
     cases = []
