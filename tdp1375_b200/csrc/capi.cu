@@ -71,6 +71,7 @@ int tdp_destroy_slots(void) {
     }
     try {
         old.clear();
+        tdp::pi_filter_release();
     } catch (const std::exception &e) {
         return map_exception(e);
     }
