@@ -87,7 +87,9 @@ struct alignas(128) EngineCtl {
     int stop;  // line 3: launch stop + error
     int error;
     int pad3[30];
-    unsigned long long stats[kStatCount];  // line 4
+    int idle;  // line 4: registered idle warps not yet claimed by a donor
+    int pad4[31];
+    unsigned long long stats[kStatCount];  // line 5
 };
 
 // Per-warp mailbox: a donor that dequeued this warp from the idle ring writes a Task here
