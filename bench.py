@@ -547,8 +547,8 @@ def extra_pi_filter(native):
             rec["reference_rows"] = len(ref_rows)
             rec["call_speedup_over_reference"] = round(min(rw) / min(walls), 2)
         out[f"n{n}"] = rec
-    out["note"] = ("kernel_ms: count, scan and write kernels of tdp_pi_filter (packed 4-bit registers, n <= 16); "
-                   "call_ms includes its allocations and copies, like reference_call_ms (performGpuPiFilter, "
+    out["note"] = ("kernel_ms: count and write kernels of tdp_pi_filter (120 candidates per thread as bits, n <= 16); "
+                   "call_ms includes its copies, like reference_call_ms (performGpuPiFilter, "
                    "oracle/_ref); the filter is ALU-bound (candidates generated on chip, hits written)")
     return out
 

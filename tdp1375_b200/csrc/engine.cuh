@@ -51,7 +51,7 @@ struct alignas(16) Task {
     uint8_t reserved1;
     uint16_t lo;
     uint16_t hi;
-    uint32_t flags;                  // bit 0: unexpanded node; bits 8..15: first-level rank + 1
+    uint32_t flags;                  // bit 0: unexpanded node; bit 1: share eagerly; bits 8..15: first-level rank + 1
     uint32_t path[16];
     uint8_t spi[64];
     uint8_t pi[64];
@@ -165,6 +165,7 @@ struct EngineParams {
     int maxInFlight;                 // admitted-but-unfinished instance cap (0 = none)
     int replace;                     // full-window policy: 0 admit unrecorded, 1 deepest, 2 oldest,
                                      // 3 deepest then oldest (see dedup_admit_warp)
+    int eager;                       // 1: few instances, share work after every chunk while most warps wait
     int commute;                     // 1: partial-order reduction of commuting moves (por_skip)
     int probeLeaves;                 // 1: probe the table for children whose children are leaves
 };

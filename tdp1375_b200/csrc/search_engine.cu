@@ -224,6 +224,7 @@ void SearchSlot::dropGraph() {
 
 int SearchSlot::stage(const tdp_instance *instances, int count, float minRate, std::string &err) {
     graphValid_ = false;
+    resultsRead_ = false;
     order_.clear();
     order_.reserve(count);
     for (int pass = 0; pass < 2; ++pass)
@@ -291,14 +292,6 @@ int SearchSlot::stage(const tdp_instance *instances, int count, float minRate, s
 
 void SearchSlot::launchClass(int cls, int offset, int count) {
     if (count <= 0) return;
-    // the generation word is copied from hGen_[cls], which runStaged set before this run
-    check(cudaMemcpyAsync(dGen_, hGen_ + cls, sizeof(uint32_t), cudaMemcpyHostToDevice, stream_), "generation");
-    check(cudaMemsetAsync(dCtl_, 0, sizeof(EngineCtl), stream_), "reset ctl");
-    check(cudaMemsetAsync(dOut_ + offset, 0, (size_t)count * sizeof(InstanceOut), stream_), "reset results");
-    check(cudaMemsetAsync(dDone_, 0, (size_t)((count + 31) / 32) * sizeof(uint32_t), stream_), "reset done bits");
-    check(cudaMemsetAsync(dMail_, 0, (size_t)mailboxes_ * sizeof(Mailbox), stream_), "reset mailboxes");
-    check(cudaMemsetAsync(dRing_, 0, (size_t)ringSize_ * sizeof(uint32_t), stream_), "reset idle ring");
-
     EngineParams P{};
     P.in = dIn_ + offset;
     P.out = dOut_ + offset;
@@ -336,9 +329,16 @@ void SearchSlot::launchClass(int cls, int offset, int count) {
     blocksPerSM = std::max(1, blocksPerSM);
     // every warp of the grid needs a mailbox
     const int grid = std::min(numSMs_ * blocksPerSM, mailboxes_ / dev::kWarpsPerBlock);
+    P.eager = (int64_t)count * dev::kEagerWarps <= (int64_t)grid * dev::kWarpsPerBlock;
     P.maxInFlight = cfg_.warps_per_instance > 0
                         ? std::max(1, grid * dev::kWarpsPerBlock / cfg_.warps_per_instance)
                         : 0;
+    // the generation word is read from hGen_[cls], which runStaged set before this run
+    const int resetBlocks = std::min(numSMs_, std::max(16, (count * (int)(sizeof(InstanceOut) / 16) + 255) / 256));
+    dev::reset_kernel<<<resetBlocks, 256, 0, stream_>>>(dCtl_, dOut_ + offset, count, dDone_, dMail_, mailboxes_, dRing_,
+                                                        dRing_ + ringSize_, (int)ringSize_, grid * dev::kWarpsPerBlock,
+                                                        dGen_, hGen_ + cls);
+    check(cudaGetLastError(), "launch reset_kernel");
     kernel<<<grid, threads, smem, stream_>>>(P);
     check(cudaGetLastError(), "launch search_engine_kernel");
     check(cudaMemcpyAsync(hCtl_ + cls, dCtl_, sizeof(EngineCtl), cudaMemcpyDeviceToHost, stream_), "read ctl");
@@ -348,12 +348,16 @@ void SearchSlot::launchClass(int cls, int offset, int count) {
 
 // Waits for the slot stream while honouring the host cancel request (the device flag
 // was already written by cancel()).
+// A sleep of 20 us takes about 75 us, a third of a small search's time, so the first
+// half millisecond is polled without.
 void SearchSlot::wait() {
+    const auto start = std::chrono::steady_clock::now();
     while (true) {
         const cudaError_t q = cudaStreamQuery(stream_);
         if (q == cudaSuccess) return;
         if (q != cudaErrorNotReady) check(q, "search kernel");
-        std::this_thread::sleep_for(std::chrono::microseconds(20));
+        if (std::chrono::steady_clock::now() - start > std::chrono::microseconds(500))
+            std::this_thread::sleep_for(std::chrono::microseconds(20));
     }
 }
 
@@ -374,6 +378,7 @@ int SearchSlot::runStaged(std::string &err) {
     check(cudaSetDevice(device_), "cudaSetDevice");
     deviceError_ = 0;
     launches_ = 0;
+    resultsRead_ = false;
     std::fill(std::begin(statsAccum_), std::end(statsAccum_), 0ull);
     // Table generations: one per size class per run.  On wrap-around, or when the entry
     // layout changes, the table is cleared (outside any graph).
@@ -419,7 +424,12 @@ int SearchSlot::runStaged(std::string &err) {
         if (rc != 0) return rc;
     }
     check(cudaEventRecord(evStop_, stream_), "event");
+    // the results come back with the run: no second round trip in fetch
+    if (count_ > 0)
+        check(cudaMemcpyAsync(hOut_, dOut_, (size_t)count_ * sizeof(InstanceOut), cudaMemcpyDeviceToHost, stream_),
+              "read results");
     wait();
+    resultsRead_ = true;
     for (int cls = 0; cls < 2; ++cls) {
         if (!launched_[cls]) continue;
         const EngineCtl &c = hCtl_[cls];
@@ -448,7 +458,7 @@ int SearchSlot::runStaged(std::string &err) {
 
 int SearchSlot::fetch(tdp_result *results) {
     check(cudaSetDevice(device_), "cudaSetDevice");
-    if (count_ > 0) {
+    if (count_ > 0 && !resultsRead_) {
         check(cudaMemcpyAsync(hOut_, dOut_, (size_t)count_ * sizeof(InstanceOut), cudaMemcpyDeviceToHost, stream_),
               "read results");
         check(cudaStreamSynchronize(stream_), "sync results");

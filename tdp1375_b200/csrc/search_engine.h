@@ -101,8 +101,9 @@ private:
 
     std::vector<int> order_;
     int count_ = 0, countSmall_ = 0;
+    bool resultsRead_ = false;  // hOut_ holds the last run's results
 
-    tdp_engine_config cfg_{0, 8, 1, 0, 120.0, 2, 0, 0, 2, 1, 0};
+    tdp_engine_config cfg_{0, 16, 1, 0, 120.0, 2, 0, 0, 2, 1, 0};
     unsigned long long statsAccum_[kStatCount] = {};
     double kernelMs_ = 0.0;
     int deviceError_ = 0;

@@ -46,6 +46,7 @@ namespace dev {
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kWarpsPerBlock = 8;
 constexpr int kSpinLimit = 1 << 20;
+constexpr uint32_t kFlagCycles = 2000;
 
 template <int NW>
 struct KeyTraits;
@@ -445,10 +446,8 @@ __device__ __forceinline__ bool por_skip(uint32_t inc, uint32_t x, uint32_t y, u
 // or about to be.  A compare-and-swap of the head let one donor through per round trip, all
 // others retrying: 1.2 to 1.7 donations per microsecond on the whole chip whatever the poll
 // interval, and 30 % of the warps waited at 64 chunks per poll, 60 % at 4.  With the tickets 2 %
-// wait at 8 chunks per poll (the default, 64 before): 1,000 exhaustive searches of 4..6
-// 3-cycles take 182 ms instead of 228 ms (180 to 186 ms from 4 to 64 chunks), the largest 8-cycle
-// cases 245 ms instead of 306 ms, and 8 staged single searches, where the poll interval is the
-// time until a second warp has work, 5.2 to 8.0 ms instead of 11.8 to 20.1 ms.
+// wait at 16 chunks per poll (the default, 64 before): 1,000 exhaustive searches of 4..6
+// 3-cycles take 186 ms instead of 228 ms and the largest 8-cycle cases 235 ms instead of 306 ms.
 __device__ __forceinline__ void ring_failed(const EngineParams &P) {
     atomicExch(&P.ctl->error, kErrSpinLimit);
     atomicExch(&P.ctl->stop, 1);
@@ -489,6 +488,9 @@ __device__ __forceinline__ int ring_dequeue(const EngineParams &P) {
     ring_failed(P);
     return -1;
 }
+
+constexpr uint32_t kTaskEager = 2u;  // Task::flags: the donor saw most warps waiting
+constexpr int kEagerShares = 8, kEagerWarps = 64;
 
 // Children words (spi/pi fields only; tables are rebuilt by the caller) of the move that
 // takes positions (i, j, k), i.e. symbols a, b, c with cycle words wa, wb, wc.
@@ -753,6 +755,35 @@ struct WarpShared {
     unsigned long long stats[kStatCount];  // per-warp counters, flushed once at exit
 };
 
+// Clears what a launch starts from: control block, results, done bits, the mailbox flags of its
+// warps and the ring; reads the table generation from pinned host memory.  One launch of a few
+// microseconds instead of five memsets and a copy.  Warps beyond the number of instances find
+// themselves registered in the ring: thousands of registrations at once are as many atomics on
+// two words.
+__global__ void __launch_bounds__(256) reset_kernel(EngineCtl *ctl, InstanceOut *out, int count, uint32_t *doneBits,
+                                                    Mailbox *mail, int mailboxes, uint32_t *ringSeq, uint32_t *ringWid,
+                                                    int ringSize, int warps, uint32_t *generation,
+                                                    const uint32_t *hostGeneration) {
+    const int first = (int)(blockIdx.x * blockDim.x + threadIdx.x), step = (int)(gridDim.x * blockDim.x);
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    if (first == 0) *generation = *reinterpret_cast<const volatile uint32_t *>(hostGeneration);
+    const int waiting = max(0, warps - count);  // warps without a first instance start in the ring
+    for (int i = first; i < (int)(sizeof(EngineCtl) / sizeof(uint4)); i += step) {
+        uint4 v = zero;
+        if (i == (int)(offsetof(EngineCtl, ringTail) / sizeof(uint4))) v.x = (uint32_t)waiting;
+        if (i == (int)(offsetof(EngineCtl, idle) / sizeof(uint4))) v.x = (uint32_t)waiting;
+        reinterpret_cast<uint4 *>(ctl)[i] = v;
+    }
+    const int64_t words = (int64_t)count * (int64_t)(sizeof(InstanceOut) / sizeof(uint4));
+    for (int64_t i = first; i < words; i += step) reinterpret_cast<uint4 *>(out)[i] = zero;
+    for (int i = first; i < (count + 31) / 32; i += step) doneBits[i] = 0u;
+    for (int i = first; i < mailboxes; i += step) mail[i].flag = 0u;
+    for (int i = first; i < ringSize; i += step) {
+        ringSeq[i] = i < waiting ? 1u : 0u;
+        if (i < waiting) ringWid[i] = (uint32_t)(count + i);
+    }
+}
+
 template <int NW>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_engine_kernel(const EngineParams P) {
     using K = KeyTraits<NW>;
@@ -765,15 +796,22 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
     const unsigned long long deadline = global_time_ns() + P.timeLimitNs;
     const uint32_t generation = __ldcg(P.generation);
 
+    // Idle warps of a block look at the launch's flags in turn, one every kFlagCycles, and learn of
+    // its end from one another: thousands of warps reading four words slowed the warps at work.
+    __shared__ volatile int blockOver;
+    __shared__ volatile uint32_t blockLook;
+    if (threadIdx.x == 0) {
+        blockOver = 0;
+        blockLook = (uint32_t)clock64();
+    }
     if (lane < kStatCount) S.stats[lane] = 0ull;
-    __syncwarp();
+    __syncthreads();
     const uint32_t gw = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    bool registered = false;
+    bool registered = gw >= (uint32_t)P.count;  // reset_kernel has entered those
     int backoff = 64;
     // Busy and lifetime cycles accumulate in the warp's shared counters (start times are
     // subtracted, end times added; unsigned arithmetic wraps back), so no register stays live.
     if (lane == 0) S.stats[kStatWarpCycles] -= (unsigned long long)clock64();
-    int idleRound = 0;
     bool stopAll = false;
 
     while (!stopAll) {
@@ -784,8 +822,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
         if (lane == 0) {
             if (registered && ld_acquire_u32(&P.mail[gw].flag) != 0u) kind = 1;
             if (kind == 0) {
-                const bool full = registered ? ((++idleRound & 7) == 0) : true;
-                if (full) {
+                bool full = true;
+                if (registered) {
+                    const uint32_t now = (uint32_t)clock64();
+                    full = now - blockLook > kFlagCycles;
+                    if (full) blockLook = now;
+                    if (blockOver) kind = -1;
+                }
+                if (full && kind == 0) {
                     const int stopFlag = ld_relaxed_s32(&ctl->stop);
                     const int cancelFlag = ld_relaxed_s32(P.cancel);
                     const bool late = global_time_ns() > deadline;
@@ -820,6 +864,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                     }
                 }
                 if (kind == 0 && full && ld_relaxed_s32(&ctl->doneCount) >= P.count) kind = -1;
+                if (kind < 0) blockOver = 1;
             }
         }
         kind = __shfl_sync(kFull, kind, 0);
@@ -831,7 +876,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
             continue;
         }
         backoff = 64;
-        idleRound = 0;
         if (lane == 0) S.stats[kStatBusyCycles] -= (unsigned long long)clock64();
 
         // ---------------------------------------------------------------- set up
@@ -950,7 +994,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
             if (lane == 0) st = ld_relaxed_s32(&P.out[inst].state);
             if (__shfl_sync(kFull, st, 0) == kStateFound) outcome = 1;
         }
-        int poll = 0;
+        // Chunks until the next poll.  In a launch of few instances (P.eager: at least kEagerWarps
+        // warps for each) and while more than half of the warps wait, a warp polls after every chunk and
+        // hands out up to kEagerShares pieces at once, and so do the warps it gives work to: the time
+        // until the chip is busy is the chain of first donations (12 staged searches of the combination
+        // step's configurations: 9.5 ms at 16 chunks per poll, 5.9 ms so).  With more instances it
+        // would only cut the work into smaller pieces (1,000 searches: 2 % slower at 4 chunks per poll).
+        int poll = P.eager && (kind == 2 || (S.staging[3] & kTaskEager)) ? 1 : P.pollInterval;
         while (outcome == 0) {
             if (pending == 0u) {
                 if (cursor >= end) {
@@ -974,8 +1024,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                     sf = sparse_setup<NW>(w, n, lane, even, satMask, expMask, ordered(f) ? 0 : P.sparse, S.tri, S.cycles);
                     continue;
                 }
-                if (++poll >= P.pollInterval) {
-                    poll = 0;
+                if (--poll <= 0) {
                     int act = 0;
                     if (lane == 0) {
                         // Independent loads, issued together: one L2 round trip per poll.
@@ -995,13 +1044,17 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                         } else if (idle > 0) {
                             act = 3;
                         }
+                        if (P.eager && 2 * idle > (int)(gridDim.x * kWarpsPerBlock)) act |= 4;
                     }
                     act = __shfl_sync(kFull, act, 0);
+                    const bool eager = act & 4;
+                    poll = eager ? 1 : P.pollInterval;
+                    act &= 3;
                     if (act == 1 || act == 2) {
                         outcome = act;
                         break;
                     }
-                    if (act == 3) {
+                    for (int shares = act != 3 ? 0 : eager ? kEagerShares : 1; shares > 0; --shares) {
                         // ------------------------------------------------ donate
                         // Candidates: the shallowest frame with >= 2 unevaluated chunks
                         // (split its range), or a shallower frame holding admitted children
@@ -1038,7 +1091,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                         int target = -1;
                         if (mode != 0 && lane == 0) target = ring_dequeue(P);
                         target = __shfl_sync(kFull, target, 0);
-                        if (target >= 0) {
+                        if (target < 0) break;
+                        {
                             Task *tk = &P.mail[target].task;
                             const int gEven = (g == f) ? even : S.frames[g].even;
                             uint32_t hdr1, hdr2, hdr3;
@@ -1128,7 +1182,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                                 hdr[0] = inst;
                                 hdr[1] = hdr1;
                                 hdr[2] = hdr2;
-                                hdr[3] = hdr3;
+                                hdr[3] = hdr3 | (eager ? kTaskEager : 0u);
                                 atomicAdd(&P.out[inst].outstanding, 1);
                             }
                             __threadfence();
@@ -1347,21 +1401,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
     }
 
     // ---------------------------------------------------------------- statistics
-    if (lane == 0) {
-        atomicAdd(&ctl->stats[kStatNodes], S.stats[kStatNodes]);
-        atomicAdd(&ctl->stats[kStatChildren], S.stats[kStatChildren]);
-        atomicAdd(&ctl->stats[kStatDedupProbes], S.stats[kStatDedupProbes]);
-        atomicAdd(&ctl->stats[kStatDedupPruned], S.stats[kStatDedupPruned]);
-        atomicAdd(&ctl->stats[kStatDedupInserts], S.stats[kStatDedupInserts]);
-        atomicAdd(&ctl->stats[kStatDedupFull], S.stats[kStatDedupFull]);
-        atomicAdd(&ctl->stats[kStatDonations], S.stats[kStatDonations]);
-        atomicAdd(&ctl->stats[kStatTaskPops], S.stats[kStatTaskPops]);
-        atomicAdd(&ctl->stats[kStatDedupReplaced], S.stats[kStatDedupReplaced]);
-        atomicAdd(&ctl->stats[kStatTableAtomics], S.stats[kStatTableAtomics]);
-        atomicAdd(&ctl->stats[kStatCommuteSkips], S.stats[kStatCommuteSkips]);
-        S.stats[kStatWarpCycles] += (unsigned long long)clock64();
-        atomicAdd(&ctl->stats[kStatBusyCycles], S.stats[kStatBusyCycles]);
-        atomicAdd(&ctl->stats[kStatWarpCycles], S.stats[kStatWarpCycles]);
+    // One add per counter and block: one per warp, all on one line, took tens of microseconds.
+    if (lane == 0) S.stats[kStatWarpCycles] += (unsigned long long)clock64();
+    __syncthreads();
+    if (threadIdx.x < kStatCount) {
+        unsigned long long sum = 0ull;
+        for (int q = 0; q < kWarpsPerBlock; ++q) sum += smem[q].stats[threadIdx.x];
+        if (sum) atomicAdd(&ctl->stats[threadIdx.x], sum);
     }
 }
 
