@@ -333,11 +333,11 @@ void SearchSlot::launchClass(int cls, int offset, int count) {
     P.maxInFlight = cfg_.warps_per_instance > 0
                         ? std::max(1, grid * dev::kWarpsPerBlock / cfg_.warps_per_instance)
                         : 0;
+    if (P.maxInFlight >= count) P.maxInFlight = 0;
     // the generation word is read from hGen_[cls], which runStaged set before this run
     const int resetBlocks = std::min(numSMs_, std::max(16, (count * (int)(sizeof(InstanceOut) / 16) + 255) / 256));
     dev::reset_kernel<<<resetBlocks, 256, 0, stream_>>>(dCtl_, dOut_ + offset, count, dDone_, dMail_, mailboxes_, dRing_,
-                                                        dRing_ + ringSize_, (int)ringSize_, grid * dev::kWarpsPerBlock,
-                                                        dGen_, hGen_ + cls);
+                                                        (int)ringSize_, dGen_, hGen_ + cls);
     check(cudaGetLastError(), "launch reset_kernel");
     kernel<<<grid, threads, smem, stream_>>>(P);
     check(cudaGetLastError(), "launch search_engine_kernel");

@@ -453,20 +453,50 @@ __device__ __forceinline__ void ring_failed(const EngineParams &P) {
     atomicExch(&P.ctl->stop, 1);
 }
 
-__device__ __forceinline__ bool ring_enqueue(const EngineParams &P, uint32_t wid) {
-    const uint32_t pos = atomicAdd(&P.ctl->ringTail, 1u);
+// Fills the slot of an enqueue ticket; the caller then adds the id to the count.
+__device__ __forceinline__ bool ring_place(const EngineParams &P, uint32_t pos, uint32_t wid) {
     const uint32_t slot = pos & P.ringMask, lap = pos & ~P.ringMask;
     for (int it = 0; it < kSpinLimit; ++it) {
         if (ld_acquire_u32(P.ringSeq + slot) == lap) {
             P.ringWid[slot] = wid;
             st_release_u32(P.ringSeq + slot, lap + 1u);
-            atomicAdd(&P.ctl->idle, 1);
             return true;
         }
         __nanosleep(32);
     }
     ring_failed(P);
     return false;
+}
+
+__device__ __forceinline__ bool ring_enqueue(const EngineParams &P, uint32_t wid) {
+    if (!ring_place(P, atomicAdd(&P.ctl->ringTail, 1u), wid)) return false;
+    atomicAdd(&P.ctl->idle, 1);
+    return true;
+}
+
+// First work of a block that has started (its first warp calls it): the block takes the next
+// instances, one per warp, and enters its other warps in the ring.  Returns the first warp's
+// instance; a warp whose instance is past the last one waits.  Blocks take instances and enter
+// the ring only once they run, so a launch that shares the SMs with other kernels finishes with
+// the blocks it has: an id of a block that is not resident yet would be handed work that then
+// waits for the other kernels to end.  Instances and ids move 8 at a time, one atomic per block
+// on each word (a registration per warp was thousands of atomics on two words at every start).
+__device__ __forceinline__ int block_start(const EngineParams &P, int lane) {
+    EngineCtl *ctl = P.ctl;
+    int first = P.count;
+    if (lane == 0 && ld_relaxed_s32(&ctl->nextInstance) < P.count)
+        first = atomicAdd(&ctl->nextInstance, kWarpsPerBlock);
+    first = __shfl_sync(kFull, first, 0);
+    const int busy = max(0, min(P.count - first, kWarpsPerBlock)), waiting = kWarpsPerBlock - busy;
+    if (waiting > 0) {
+        uint32_t pos = 0u;
+        if (lane == 0) pos = atomicAdd(&ctl->ringTail, (uint32_t)waiting);
+        pos = __shfl_sync(kFull, pos, 0) + (uint32_t)lane;
+        const bool placed =
+            lane >= waiting || ring_place(P, pos, (uint32_t)((int)blockIdx.x * kWarpsPerBlock + busy + lane));
+        if (__all_sync(kFull, placed) && lane == 0) atomicAdd(&ctl->idle, waiting);
+    }
+    return first;
 }
 
 // Returns a registered idle warp id, or -1 when none is left.
@@ -751,6 +781,7 @@ struct WarpShared {
     uint32_t cycles[NW == 1 ? 1 : 128];          // sparse_setup's scratch
     uint64_t rules[32];                       // success (0..15) and expansion (16..31) tables of the instance
     unsigned long long taskNodes, taskChildren;  // counters of the task in hand
+    int firstInstance;                           // taken when the block started; count or more: none (left)
     int rank1;                                   // root-order rank of the current first-level node (-1: none)
     uint32_t staging[52];
     unsigned long long stats[kStatCount];  // per-warp counters, flushed once at exit
@@ -758,31 +789,20 @@ struct WarpShared {
 
 // Clears what a launch starts from: control block, results, done bits, the mailbox flags of its
 // warps and the ring; reads the table generation from pinned host memory.  One launch of a few
-// microseconds instead of five memsets and a copy.  Warps beyond the number of instances find
-// themselves registered in the ring: thousands of registrations at once are as many atomics on
-// two words.
+// microseconds instead of five memsets and a copy.
 __global__ void __launch_bounds__(256) reset_kernel(EngineCtl *ctl, InstanceOut *out, int count, uint32_t *doneBits,
-                                                    Mailbox *mail, int mailboxes, uint32_t *ringSeq, uint32_t *ringWid,
-                                                    int ringSize, int warps, uint32_t *generation,
-                                                    const uint32_t *hostGeneration) {
+                                                    Mailbox *mail, int mailboxes, uint32_t *ringSeq, int ringSize,
+                                                    uint32_t *generation, const uint32_t *hostGeneration) {
     const int first = (int)(blockIdx.x * blockDim.x + threadIdx.x), step = (int)(gridDim.x * blockDim.x);
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     if (first == 0) *generation = *reinterpret_cast<const volatile uint32_t *>(hostGeneration);
-    const int waiting = max(0, warps - count);  // warps without a first instance start in the ring
-    for (int i = first; i < (int)(sizeof(EngineCtl) / sizeof(uint4)); i += step) {
-        uint4 v = zero;
-        if (i == (int)(offsetof(EngineCtl, ringTail) / sizeof(uint4))) v.x = (uint32_t)waiting;
-        if (i == (int)(offsetof(EngineCtl, idle) / sizeof(uint4))) v.x = (uint32_t)waiting;
-        reinterpret_cast<uint4 *>(ctl)[i] = v;
-    }
+    for (int i = first; i < (int)(sizeof(EngineCtl) / sizeof(uint4)); i += step)
+        reinterpret_cast<uint4 *>(ctl)[i] = zero;
     const int64_t words = (int64_t)count * (int64_t)(sizeof(InstanceOut) / sizeof(uint4));
     for (int64_t i = first; i < words; i += step) reinterpret_cast<uint4 *>(out)[i] = zero;
     for (int i = first; i < (count + 31) / 32; i += step) doneBits[i] = 0u;
     for (int i = first; i < mailboxes; i += step) mail[i].flag = 0u;
-    for (int i = first; i < ringSize; i += step) {
-        ringSeq[i] = i < waiting ? 1u : 0u;
-        if (i < waiting) ringWid[i] = (uint32_t)(count + i);
-    }
+    for (int i = first; i < ringSize; i += step) ringSeq[i] = 0u;
 }
 
 template <int NW>
@@ -806,9 +826,17 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
         blockLook = (uint32_t)clock64();
     }
     if (lane < kStatCount) S.stats[lane] = 0ull;
+    // With a cap on the instances in flight every warp asks for itself, below.
+    __shared__ int blockFirst;
+    if (threadIdx.x < 32) {
+        const int first = P.maxInFlight > 0 ? P.count : block_start(P, lane);
+        if (lane == 0) blockFirst = first;
+    }
     __syncthreads();
     const uint32_t gw = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    bool registered = gw >= (uint32_t)P.count;  // reset_kernel has entered those
+    if (lane == 0) S.firstInstance = blockFirst + (int)(threadIdx.x >> 5);
+    // block_start has entered the warps without an instance
+    bool registered = P.maxInFlight <= 0 && blockFirst + (int)(threadIdx.x >> 5) >= P.count;
     int backoff = 64;
     // Busy and lifetime cycles accumulate in the warp's shared counters (start times are
     // subtracted, end times added; unsigned arithmetic wraps back), so no register stays live.
@@ -840,7 +868,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                     }
                     if ((stopFlag | cancelFlag) || late) kind = -1;
                 }
-                if (kind == 0 && !registered) {
+                if (kind == 0 && S.firstInstance < P.count) {
+                    kind = 2;
+                    idx = S.firstInstance;
+                    S.firstInstance = P.count;
+                } else if (kind == 0 && !registered) {
                     // With a cap, a warp admits only while fewer than maxInFlight admitted
                     // instances are unfinished (a racy check: the cap may be exceeded by the
                     // few warps that pass it together); otherwise it registers as a helper.
