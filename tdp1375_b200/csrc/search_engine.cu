@@ -230,6 +230,9 @@ int SearchSlot::stage(const tdp_instance *instances, int count, float minRate, s
     for (int pass = 0; pass < 2; ++pass)
         for (int i = 0; i < count; ++i)
             if ((instances[i].n > 32) == (pass == 1)) order_.push_back(i);
+    exhaustive_[0] = exhaustive_[1] = false;
+    for (int i = 0; i < count; ++i)
+        if (instances[i].full_sorting) exhaustive_[instances[i].n <= 32 ? 0 : 1] = true;
     countSmall_ = 0;
     for (int i = 0; i < count; ++i) countSmall_ += instances[i].n <= 32 ? 1 : 0;
     count_ = count;
@@ -290,13 +293,29 @@ int SearchSlot::stage(const tdp_instance *instances, int count, float minRate, s
     return 0;
 }
 
+// Chunks between two polls of a busy warp when the configuration leaves it to the launch.  A
+// search that must be exhausted visits the same nodes however it is shared, so it is shared
+// early.  One that stops at its first sequence visits the more nodes the wider its front, and the
+// nearer the instances come to one per warp, the less sharing buys.  20,000 searches of 8..10
+// 3-cycles, partial mode, one B200, device time at 16 / 32 / 64 / 128 chunks per poll, by
+// instances in a launch (4,736 warps):
+//    1,000  1,377 / 1,408 / 1,372 / 1,445 ms      3,000  2,477 / 2,190 / 2,084 / 1,958 ms
+//    1,500  1,836 / 1,796 / 1,684 / 1,650        10,000  3,652 / 3,537 / 3,354 / 3,185
+//    2,000  2,349 / 2,153 / 1,994 / 1,943        20,000  4,815 / 4,696 / 4,655 / 4,484
+// (nodes in proportion; 256 is no better than 128).  2,000 searches under the learned order, which
+// end sooner: 52 / 51 / 52 / 57 ms; hence the step at 64.  Full sortings of 4..6 3-cycles, 1,000 in
+// a launch: 268 ms per 4,000 at 16, 322 at 64.
+constexpr int kDefaultPoll = 16;
+static int wide_poll(int64_t inFlight, int64_t warps) {
+    return 2 * inFlight >= warps ? 128 : 4 * inFlight >= warps ? 64 : kDefaultPoll;
+}
+
 void SearchSlot::launchClass(int cls, int offset, int count) {
     if (count <= 0) return;
     EngineParams P{};
     P.in = dIn_ + offset;
     P.out = dOut_ + offset;
     P.count = count;
-    P.pollInterval = std::max(1, cfg_.poll_interval);
     P.rules = dRules_;
     P.triples = triples_;
     P.table = dTable_;
@@ -334,6 +353,10 @@ void SearchSlot::launchClass(int cls, int offset, int count) {
                         ? std::max(1, grid * dev::kWarpsPerBlock / cfg_.warps_per_instance)
                         : 0;
     if (P.maxInFlight >= count) P.maxInFlight = 0;
+    const int inFlight = P.maxInFlight > 0 ? P.maxInFlight : count;
+    P.pollInterval = cfg_.poll_interval;
+    if (P.pollInterval == kDefaultPoll && !exhaustive_[cls])
+        P.pollInterval = wide_poll((int64_t)inFlight, (int64_t)grid * dev::kWarpsPerBlock);
     // the generation word is read from hGen_[cls], which runStaged set before this run
     const int resetBlocks = std::min(numSMs_, std::max(16, (count * (int)(sizeof(InstanceOut) / 16) + 255) / 256));
     dev::reset_kernel<<<resetBlocks, 256, 0, stream_>>>(dCtl_, dOut_ + offset, count, dDone_, dMail_, mailboxes_, dRing_,

@@ -101,6 +101,7 @@ private:
 
     std::vector<int> order_;
     int count_ = 0, countSmall_ = 0;
+    bool exhaustive_[2] = {false, false};  // per size class: some instance asks for full sorting
     bool resultsRead_ = false;  // hOut_ holds the last run's results
 
     tdp_engine_config cfg_{0, 16, 1, 0, 120.0, 2, 0, 0, 2, 1, 0};
