@@ -31,6 +31,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "mlp.h"
 
@@ -402,15 +403,24 @@ int launch(int form, int bn, int splits, CUtensorMap &ma, CUtensorMap &mb, CUten
 }  // namespace
 
 int prepare(std::string &err) {
-    static std::once_flag attrOnce;
-    static cudaError_t attrErr = cudaSuccess;
-    std::call_once(attrOnce, [] {
-        for (int f = 0; f < kForms && attrErr == cudaSuccess; ++f)
-            attrErr = cudaFuncSetAttribute(kKernels[f], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           std::max(smem_bytes(64), smem_bytes(128)));
-    });
-    if (attrErr != cudaSuccess) {
-        err = std::string("gemm set-up: ") + cudaGetErrorString(attrErr);
+    // a kernel's shared-memory limit is raised on each device by itself
+    static std::mutex mu;
+    static std::vector<bool> raised;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (e == cudaSuccess && (size_t)device >= raised.size()) raised.resize((size_t)device + 1, false);
+        if (e == cudaSuccess && !raised[(size_t)device]) {
+            for (int f = 0; f < kForms && e == cudaSuccess; ++f)
+                e = cudaFuncSetAttribute(kKernels[f], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         std::max(smem_bytes(64), smem_bytes(128)));
+            raised[(size_t)device] = e == cudaSuccess;
+        }
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here, not by the next launch's check
+        err = std::string("gemm set-up: ") + cudaGetErrorString(e);
         return -3;
     }
     return encode_fn(err) ? 0 : -1;
