@@ -474,29 +474,15 @@ __device__ __forceinline__ bool ring_enqueue(const EngineParams &P, uint32_t wid
     return true;
 }
 
-// First work of a block that has started (its first warp calls it): the block takes the next
-// instances, one per warp, and enters its other warps in the ring.  Returns the first warp's
-// instance; a warp whose instance is past the last one waits.  Blocks take instances and enter
-// the ring only once they run, so a launch that shares the SMs with other kernels finishes with
-// the blocks it has: an id of a block that is not resident yet would be handed work that then
-// waits for the other kernels to end.  Instances and ids move 8 at a time, one atomic per block
-// on each word (a registration per warp was thousands of atomics on two words at every start).
-__device__ __forceinline__ int block_start(const EngineParams &P, int lane) {
-    EngineCtl *ctl = P.ctl;
-    int first = P.count;
-    if (lane == 0 && ld_relaxed_s32(&ctl->nextInstance) < P.count)
-        first = atomicAdd(&ctl->nextInstance, kWarpsPerBlock);
-    first = __shfl_sync(kFull, first, 0);
-    const int busy = max(0, min(P.count - first, kWarpsPerBlock)), waiting = kWarpsPerBlock - busy;
-    if (waiting > 0) {
-        uint32_t pos = 0u;
-        if (lane == 0) pos = atomicAdd(&ctl->ringTail, (uint32_t)waiting);
-        pos = __shfl_sync(kFull, pos, 0) + (uint32_t)lane;
-        const bool placed =
-            lane >= waiting || ring_place(P, pos, (uint32_t)((int)blockIdx.x * kWarpsPerBlock + busy + lane));
-        if (__all_sync(kFull, placed) && lane == 0) atomicAdd(&ctl->idle, waiting);
-    }
-    return first;
+// Enters the block's warps from `busy` on in the ring; their last one calls it.
+__device__ __forceinline__ void ring_enter_block(const EngineParams &P, int busy, int lane) {
+    const int waiting = kWarpsPerBlock - busy;
+    uint32_t pos = 0u;
+    if (lane == 0) pos = atomicAdd(&P.ctl->ringTail, (uint32_t)waiting);
+    pos = __shfl_sync(kFull, pos, 0) + (uint32_t)lane;
+    const bool placed =
+        lane >= waiting || ring_place(P, pos, (uint32_t)((int)blockIdx.x * kWarpsPerBlock + busy + lane));
+    if (__all_sync(kFull, placed) && lane == 0) atomicAdd(&P.ctl->idle, waiting);
 }
 
 // Returns a registered idle warp id, or -1 when none is left.
@@ -826,17 +812,22 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
         blockLook = (uint32_t)clock64();
     }
     if (lane < kStatCount) S.stats[lane] = 0ull;
-    // With a cap on the instances in flight every warp asks for itself, below.
+    // A block that starts takes the next instances, one per warp, and its other warps enter the
+    // ring.  It does so only once it runs: a launch that shares the SMs with other kernels then
+    // finishes with the blocks it has, where an id of a block that is not resident yet would be
+    // handed work that waits for the other kernels to end.  Instances and ids move 8 at a time,
+    // one atomic per block on each word (one per warp was thousands of atomics on two words at
+    // every start), and the warps with an instance do not wait for the ring.  With a cap on the
+    // instances in flight every warp asks for itself, below.
     __shared__ int blockFirst;
-    if (threadIdx.x < 32) {
-        const int first = P.maxInFlight > 0 ? P.count : block_start(P, lane);
-        if (lane == 0) blockFirst = first;
-    }
+    if (threadIdx.x == 0)
+        blockFirst = P.maxInFlight > 0 ? P.count : atomicAdd(&ctl->nextInstance, kWarpsPerBlock);
     __syncthreads();
     const uint32_t gw = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (lane == 0) S.firstInstance = blockFirst + (int)(threadIdx.x >> 5);
-    // block_start has entered the warps without an instance
     bool registered = P.maxInFlight <= 0 && blockFirst + (int)(threadIdx.x >> 5) >= P.count;
+    if (registered && (threadIdx.x >> 5) == kWarpsPerBlock - 1)
+        ring_enter_block(P, max(0, P.count - blockFirst), lane);
     int backoff = 64;
     // Busy and lifetime cycles accumulate in the warp's shared counters (start times are
     // subtracted, end times added; unsigned arithmetic wraps back), so no register stays live.
