@@ -65,7 +65,9 @@ int tdp_cancel(int slot);
  * (jni_sorter.cu:111-150).  Visits every pi with pi[0]=0 over n symbols and keeps those where
  * oriented_triple is in cyclic order, cycle is oriented and (unless skip_2move_check) cycle
  * admits no 2-move.  Writes at most max_rows rows of n bytes to out, in lexicographic order
- * (the reference's order is arbitrary), and returns the total number of hits (< 0: error). */
+ * (the reference's order is arbitrary), and returns the total number of hits (< 0: error).
+ * Finished calls leave their device buffers for later ones, at most 8 sets, 96 MB together
+ * in a process; tdp_destroy_slots gives them back (also in a program that never made slots). */
 int64_t tdp_pi_filter(const uint8_t *cycle, int cycle_len, const uint8_t *oriented_triple, int triple_len, int n,
                       int skip_2move_check, uint8_t *out, int64_t max_rows);
 /* Device time in ms (CUDA events around its kernels) of this thread's last tdp_pi_filter call. */

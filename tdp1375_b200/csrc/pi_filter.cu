@@ -709,9 +709,10 @@ bool ok(cudaError_t e, std::string &err, const char *what) {
 
 // Device buffers, a pinned staging buffer and events of one call.  Allocating and freeing them
 // took 0.5 ms and more per call (n = 9: 0.9 ms of which the kernels were 30 us), so a finished
-// call leaves its workspace for the next: at most kIdleWorkspaces lie idle, each of at most
-// kIdleBytes, and tdp_destroy_slots frees them.  A call takes one out of the pool for itself,
-// so concurrent calls never share one.  A workspace belongs to the context it was made in
+// call leaves its workspace for the next: at most kIdleWorkspaces lie idle, of at most kIdleBytes
+// together (n = 12 with 2^20 rows takes 18 MB), and tdp_destroy_slots frees them, as does a call
+// that would otherwise run out of memory.  A call takes one out of the pool for itself, so
+// concurrent calls never share one.  A workspace belongs to the context it was made in
 // (cuCtxGetId: a device that was reset has another), and serves only calls in that context.
 constexpr size_t kIdleBytes = 96u << 20;
 constexpr size_t kIdleWorkspaces = 8;
@@ -774,7 +775,9 @@ struct WorkspaceLease {
         if (finished && ws.scratchBytes + ws.rowsBytes <= kIdleBytes) {
             ws.context = current_context();
             std::lock_guard<std::mutex> lock(gIdleMutex);
-            if (ws.context && gIdle.size() < kIdleWorkspaces) {
+            size_t bytes = ws.scratchBytes + ws.rowsBytes;
+            for (const Workspace &idle : gIdle) bytes += idle.scratchBytes + idle.rowsBytes;
+            if (ws.context && gIdle.size() < kIdleWorkspaces && bytes <= kIdleBytes) {
                 gIdle.push_back(ws);
                 return;
             }
@@ -790,8 +793,15 @@ cudaError_t reserve(void *&ptr, size_t &have, size_t bytes) {
     cudaFree(ptr);
     ptr = nullptr;
     have = 0;
-    const cudaError_t e = cudaMalloc(&ptr, bytes);
+    cudaError_t e = cudaMalloc(&ptr, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        // what idle workspaces hold must not make a call fail that fits without them
+        cudaGetLastError();
+        pi_filter_release();
+        e = cudaMalloc(&ptr, bytes);
+    }
     if (e == cudaSuccess) have = bytes;
+    else cudaGetLastError();  // reported by this call, not by the next launch's check
     return e;
 }
 
