@@ -121,8 +121,10 @@ __global__ void __launch_bounds__(kXentThreads, 6) softmax_xent_kernel(const flo
         }
     }
     const int tgt = target[r];
-    bool beaten = false;  // some logit ranks before the target's (greater, or equal and earlier)
-    if (kTop1) {
+    // some logit ranks before the target's (greater, or equal and earlier); a target that is no
+    // triple is never the greatest
+    bool beaten = tgt < 0 || tgt >= kTriples;
+    if (kTop1 && !beaten) {
         const float tv = row[tgt];
         const bool isNan = tv != tv;  // a NaN ranks as the greatest
 #pragma unroll
