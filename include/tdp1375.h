@@ -128,8 +128,7 @@ typedef struct tdp_engine_config {
     int32_t blocks_per_sm;   /* 0 = occupancy maximum */
     int32_t poll_interval;   /* chunks between flag polls / donation checks; 16 (default) leaves it to
                                 the launch: when every instance stops at its first sequence, 64 from
-                                one instance in flight per four warps on and 128 from one per two,
-                                else 16 */
+                                one instance per four warps on and 128 from one per two, else 16 */
     int32_t tight_bound;     /* 1 = verdict-preserving strengthened prune, 0 = reference prune only */
     int32_t task_capacity;   /* read-only: warp mailboxes for work donation (sized from the queue budget) */
     double time_limit_s;     /* device deadline per launch */

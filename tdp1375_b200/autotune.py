@@ -4,7 +4,8 @@ The engine's tunables and what they stand for in the batched-search design:
   * ``blocks_per_sm``      resident warps per SM, i.e. how many warps share the instances
                            (8 warps per block);
   * ``poll_interval``      chunks between a busy warp's looks at the idle-warp ring, i.e.
-                           the granularity at which work is split off and donated;
+                           the granularity at which work is split off and donated
+                           (16, the default, leaves the choice to the launch);
   * ``warps_per_instance`` grid warps per in-flight instance (0: no cap), i.e. how many
                            instances hold live table entries at once;
   * ``table_entries``      transposition-table capacity, i.e. its load for the batch;

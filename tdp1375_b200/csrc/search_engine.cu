@@ -303,11 +303,12 @@ int SearchSlot::stage(const tdp_instance *instances, int count, float minRate, s
 //    1,500  1,836 / 1,796 / 1,684 / 1,650        10,000  3,652 / 3,537 / 3,354 / 3,185
 //    2,000  2,349 / 2,153 / 1,994 / 1,943        20,000  4,815 / 4,696 / 4,655 / 4,484
 // (nodes in proportion; 256 is no better than 128).  2,000 searches under the learned order, which
-// end sooner: 52 / 51 / 52 / 57 ms; hence the step at 64.  Full sortings of 4..6 3-cycles, 1,000 in
+// end sooner: 52 / 51 / 52 / 57 ms; hence the step at 64.  A cap on the instances in flight does
+// not change this: 100,000 uneven instances at 8 warps each 1,059 / 993 / 919 / 807 ms.  Full sortings of 4..6 3-cycles, 1,000 in
 // a launch: 268 ms per 4,000 at 16, 322 at 64.
 constexpr int kDefaultPoll = 16;
-static int wide_poll(int64_t inFlight, int64_t warps) {
-    return 2 * inFlight >= warps ? 128 : 4 * inFlight >= warps ? 64 : kDefaultPoll;
+static int wide_poll(int64_t count, int64_t warps) {
+    return 2 * count >= warps ? 128 : 4 * count >= warps ? 64 : kDefaultPoll;
 }
 
 void SearchSlot::launchClass(int cls, int offset, int count) {
@@ -353,10 +354,9 @@ void SearchSlot::launchClass(int cls, int offset, int count) {
                         ? std::max(1, grid * dev::kWarpsPerBlock / cfg_.warps_per_instance)
                         : 0;
     if (P.maxInFlight >= count) P.maxInFlight = 0;
-    const int inFlight = P.maxInFlight > 0 ? P.maxInFlight : count;
     P.pollInterval = cfg_.poll_interval;
     if (P.pollInterval == kDefaultPoll && !exhaustive_[cls])
-        P.pollInterval = wide_poll((int64_t)inFlight, (int64_t)grid * dev::kWarpsPerBlock);
+        P.pollInterval = wide_poll(count, (int64_t)grid * dev::kWarpsPerBlock);
     // the generation word is read from hGen_[cls], which runStaged set before this run
     const int resetBlocks = std::min(numSMs_, std::max(16, (count * (int)(sizeof(InstanceOut) / 16) + 255) / 256));
     dev::reset_kernel<<<resetBlocks, 256, 0, stream_>>>(dCtl_, dOut_ + offset, count, dDone_, dMail_, mailboxes_, dRing_,
