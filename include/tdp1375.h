@@ -127,8 +127,9 @@ int tdp_last_stats(int slot, tdp_stats *out);
 typedef struct tdp_engine_config {
     int32_t blocks_per_sm;   /* 0 = occupancy maximum */
     int32_t poll_interval;   /* chunks between flag polls / donation checks; 16 (default) leaves it to
-                                the launch: when every instance stops at its first sequence, 64 from
-                                one instance per four warps on and 128 from one per two, else 16 */
+                                the launch: 128 when every instance stops at its first sequence and
+                                there are three for every eight warps (under a learned order one for
+                                every warp), else 16 */
     int32_t tight_bound;     /* 1 = verdict-preserving strengthened prune, 0 = reference prune only */
     int32_t task_capacity;   /* read-only: warp mailboxes for work donation (sized from the queue budget) */
     double time_limit_s;     /* device deadline per launch */

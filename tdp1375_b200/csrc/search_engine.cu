@@ -296,19 +296,22 @@ int SearchSlot::stage(const tdp_instance *instances, int count, float minRate, s
 // Chunks between two polls of a busy warp when the configuration leaves it to the launch.  A
 // search that must be exhausted visits the same nodes however it is shared, so it is shared
 // early.  One that stops at its first sequence visits the more nodes the wider its front, and the
-// nearer the instances come to one per warp, the less sharing buys.  20,000 searches of 8..10
-// 3-cycles, partial mode, one B200, device time at 16 / 32 / 64 / 128 chunks per poll, by
-// instances in a launch (4,736 warps):
-//    1,000  1,377 / 1,408 / 1,372 / 1,445 ms      3,000  2,477 / 2,190 / 2,084 / 1,958 ms
-//    1,500  1,836 / 1,796 / 1,684 / 1,650        10,000  3,652 / 3,537 / 3,354 / 3,185
-//    2,000  2,349 / 2,153 / 1,994 / 1,943        20,000  4,815 / 4,696 / 4,655 / 4,484
-// (nodes in proportion; 256 is no better than 128).  2,000 searches under the learned order, which
-// end sooner: 52 / 51 / 52 / 57 ms; hence the step at 64.  A cap on the instances in flight does
-// not change this: 100,000 uneven instances at 8 warps each 1,059 / 993 / 919 / 807 ms.  Full sortings of 4..6 3-cycles, 1,000 in
+// nearer the instances come to one per warp, the less sharing buys.  Times on one B200 (4,736
+// warps), partial mode, at 16 / 64 / 128 chunks per poll, by instances in a launch:
+//   20,000 of 8..10 3-cycles    1,000  1,377 / 1,372 / 1,445 ms    2,000  2,349 / 1,994 / 1,943
+//                               3,000  2,477 / 2,084 / 1,958      10,000  3,652 / 3,354 / 3,185
+//   one launch of 3..10         1,500  41 / 45 / 48                2,000  48 / 44 / 47
+//                               3,000  101 / 85 / 82               5,000  234 / 213 / 206
+//   under the learned order     2,000  57 / 61 / 65                3,000  35 / 39 / 43
+//   (3..10)                     5,000  114 / 113 / 114             8,000  213 / 196 / 189
+// (32 lies between 16 and 64, 256 is no better than 128; nodes in proportion to the times).
+// Searches under the learned order end sooner, so few of them are left for the waiting warps: the
+// line is where every warp has one.  A cap on the instances in flight does not move it: 100,000
+// uneven instances at 8 warps each 1,059 / 919 / 807 ms.  Full sortings of 4..6 3-cycles, 1,000 in
 // a launch: 268 ms per 4,000 at 16, 322 at 64.
-constexpr int kDefaultPoll = 16;
-static int wide_poll(int64_t count, int64_t warps) {
-    return 2 * count >= warps ? 128 : 4 * count >= warps ? 64 : kDefaultPoll;
+constexpr int kDefaultPoll = 16, kWidePoll = 128;
+static int launch_poll(int64_t count, int64_t warps, bool exhaustive, bool ordered) {
+    return !exhaustive && (ordered ? count >= warps : 8 * count >= 3 * warps) ? kWidePoll : kDefaultPoll;
 }
 
 void SearchSlot::launchClass(int cls, int offset, int count) {
@@ -355,8 +358,8 @@ void SearchSlot::launchClass(int cls, int offset, int count) {
                         : 0;
     if (P.maxInFlight >= count) P.maxInFlight = 0;
     P.pollInterval = cfg_.poll_interval;
-    if (P.pollInterval == kDefaultPoll && !exhaustive_[cls])
-        P.pollInterval = wide_poll(count, (int64_t)grid * dev::kWarpsPerBlock);
+    if (P.pollInterval == kDefaultPoll)
+        P.pollInterval = launch_poll(count, (int64_t)grid * dev::kWarpsPerBlock, exhaustive_[cls], P.order != nullptr);
     // the generation word is read from hGen_[cls], which runStaged set before this run
     const int resetBlocks = std::min(numSMs_, std::max(16, (count * (int)(sizeof(InstanceOut) / 16) + 255) / 256));
     dev::reset_kernel<<<resetBlocks, 256, 0, stream_>>>(dCtl_, dOut_ + offset, count, dDone_, dMail_, mailboxes_, dRing_,
