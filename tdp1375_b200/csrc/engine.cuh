@@ -156,7 +156,7 @@ struct EngineParams {
     EngineCtl *ctl;
     const int *cancel;        // slot cancel flag (device)
     unsigned long long timeLimitNs;  // every warp stops (error kErrDeadline) after this long
-    int sparse;                      // same-cycle pair enumeration allowed (n <= 32)
+    int sparse;                      // restricted enumerations: 0 none, 1 same-cycle pairs, 2 also triples
     const uint16_t *order;           // per-instance root child order (learned), or null
     int orderStride;
     const uint16_t *order2;          // per (instance, root rank < order2Ranks): best children of

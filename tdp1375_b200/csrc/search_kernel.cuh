@@ -23,10 +23,11 @@
 //     cycle length) so a child's odd-cycle count is an O(1) delta (tdp_math.cuh) instead
 //     of an O(n) recount, and a descent rebuilds the cycle tables with pointer jumping
 //     over warp shuffles;
-//   * once every instance is admitted, an idle warp registers its id in a lock-free ring and
-//     polls only its own mailbox line; a busy warp that sees waiting warps dequeues one and
-//     writes a Task straight into its mailbox: half the unexplored range of its shallowest
-//     frame, or an admitted child it has not descended into yet (work donation);
+//   * once every instance is admitted, an idle warp registers its id in a ring and polls only
+//     its own mailbox line (a block that starts registers its warps without an instance at
+//     once); a busy warp that sees waiting warps dequeues one and writes a Task straight into
+//     its mailbox: half the unexplored range of its shallowest frame, or an admitted child it
+//     has not descended into yet (work donation);
 //   * an instance ends when its last task finishes (outstanding counter), so there is
 //     no global termination scan and no queue to overflow;
 //   * the pruning rule is looked up in host-built bit tables (exact float32 semantics);
@@ -47,6 +48,7 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kWarpsPerBlock = 8;
 constexpr int kSpinLimit = 1 << 20;
 constexpr uint32_t kFlagCycles = 2000;
+constexpr int kLooks = 32;  // at some 0.7 us each
 
 template <int NW>
 struct KeyTraits;
@@ -446,8 +448,8 @@ __device__ __forceinline__ bool por_skip(uint32_t inc, uint32_t x, uint32_t y, u
 // or about to be.  A compare-and-swap of the head let one donor through per round trip, all
 // others retrying: 1.2 to 1.7 donations per microsecond on the whole chip whatever the poll
 // interval, and 30 % of the warps waited at 64 chunks per poll, 60 % at 4.  With the tickets 2 %
-// wait at 16 chunks per poll (the default, 64 before): 1,000 exhaustive searches of 4..6
-// 3-cycles take 186 ms instead of 228 ms and the largest 8-cycle cases 235 ms instead of 306 ms.
+// wait at 16 chunks per poll (the default for exhaustive searches, 64 before): 1,000 of 4..6
+// 3-cycles took 186 ms instead of 228 ms and the largest 8-cycle cases 235 ms instead of 306 ms.
 __device__ __forceinline__ void ring_failed(const EngineParams &P) {
     atomicExch(&P.ctl->error, kErrSpinLimit);
     atomicExch(&P.ctl->stop, 1);
@@ -812,22 +814,38 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
         blockLook = (uint32_t)clock64();
     }
     if (lane < kStatCount) S.stats[lane] = 0ull;
-    // A block that starts takes the next instances, one per warp, and its other warps enter the
-    // ring.  It does so only once it runs: a launch that shares the SMs with other kernels then
+    // The first blocks take an instance per warp when they start, the other warps enter the ring.
+    // A block does so only once it runs: a launch that shares the SMs with other kernels then
     // finishes with the blocks it has, where an id of a block that is not resident yet would be
-    // handed work that waits for the other kernels to end.  Instances and ids move 8 at a time,
-    // one atomic per block on each word (one per warp was thousands of atomics on two words at
-    // every start), and the warps with an instance do not wait for the ring.  With a cap on the
-    // instances in flight every warp asks for itself, below.
+    // handed work that waits for the other kernels to end.  For the same reason a later block that
+    // keeps finding instances there (blocks start in their order on this GPU, but nothing promises
+    // it) lets its warps ask for them, each for itself, as every warp does under a cap on the
+    // instances in flight.  Instances and ids move in one atomic per block on each word (one per
+    // warp was thousands of atomics on two words at every start), and the warps with an instance do
+    // not wait for the ring.  Eight instances to a block in block order is one such block per SM:
+    // taken by whichever blocks start first they crowded on few SMs (992 searches of four 3-cycles:
+    // 1,456 us per call, so 1,342); one or two to every block made each SM fetch the loop for itself
+    // (299 small searches: 314 us on the device, so 305).
     __shared__ int blockFirst;
-    if (threadIdx.x == 0)
-        blockFirst = P.maxInFlight > 0 ? P.count : atomicAdd(&ctl->nextInstance, kWarpsPerBlock);
+    const int own = (int)(threadIdx.x >> 5);
+    if (threadIdx.x == 0) {
+        int first = -1;
+        if (P.maxInFlight <= 0) {
+            if ((int)blockIdx.x * kWarpsPerBlock < P.count) {
+                first = atomicAdd(&ctl->nextInstance, kWarpsPerBlock);
+            } else {
+                for (int look = 0; look < kLooks && first < 0; ++look)
+                    if (ld_relaxed_s32(&ctl->nextInstance) >= P.count) first = P.count;
+            }
+        }
+        blockFirst = first;
+    }
     __syncthreads();
     const uint32_t gw = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    if (lane == 0) S.firstInstance = blockFirst + (int)(threadIdx.x >> 5);
-    bool registered = P.maxInFlight <= 0 && blockFirst + (int)(threadIdx.x >> 5) >= P.count;
-    if (registered && (threadIdx.x >> 5) == kWarpsPerBlock - 1)
-        ring_enter_block(P, max(0, P.count - blockFirst), lane);
+    const int busy = max(0, min(P.count - blockFirst, kWarpsPerBlock));  // (of no meaning when blockFirst < 0)
+    if (lane == 0) S.firstInstance = blockFirst < 0 ? P.count : blockFirst + own;
+    bool registered = blockFirst >= 0 && own >= busy;
+    if (registered && own == kWarpsPerBlock - 1) ring_enter_block(P, busy, lane);
     int backoff = 64;
     // Busy and lifetime cycles accumulate in the warp's shared counters (start times are
     // subtracted, end times added; unsigned arithmetic wraps back), so no register stays live.
@@ -840,7 +858,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
         // that it registers once in the idle ring and polls only its own mailbox line.
         int kind = 0, idx = 0;
         if (lane == 0) {
-            if (registered && ld_acquire_u32(&P.mail[gw].flag) != 0u) kind = 1;
+            if (S.firstInstance < P.count) {  // (the flags are read at its first poll)
+                kind = 2;
+                idx = S.firstInstance;
+                S.firstInstance = P.count;
+            } else if (registered && ld_acquire_u32(&P.mail[gw].flag) != 0u) {
+                kind = 1;
+            }
             if (kind == 0) {
                 bool full = true;
                 if (registered) {
@@ -859,11 +883,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                     }
                     if ((stopFlag | cancelFlag) || late) kind = -1;
                 }
-                if (kind == 0 && S.firstInstance < P.count) {
-                    kind = 2;
-                    idx = S.firstInstance;
-                    S.firstInstance = P.count;
-                } else if (kind == 0 && !registered) {
+                if (kind == 0 && !registered) {
                     // With a cap, a warp admits only while fewer than maxInFlight admitted
                     // instances are unfinished (a racy check: the cap may be exceeded by the
                     // few warps that pass it together); otherwise it registers as a helper.
@@ -1007,8 +1027,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
         // The frame is set up at the head of the loop, in one place for the task's first frame, a
         // return and a descent: the loop exceeds the instruction cache (4.2 of 13.9 stall cycles per
         // instruction were fetches), and three inlined copies of the set-up cost 11 % (1,000 searches
-        // of 4..6 3-cycles: 185 ms, 165 ms so; 8-cycle cases 235 ms, 209 ms so).  A donated range is in the units of its frame's mode (the receiver
-        // derives the same mode from the same node); kEndOpen covers every child.
+        // of 4..6 3-cycles: 185 ms, 165 ms so; 8-cycle cases 235 ms, 209 ms so).  A donated range is
+        // in the units of its frame's mode (the receiver derives the same mode from the same node);
+        // kEndOpen covers every child.
         SparseFrame<NW> sf;
         bool setup = true;
         if (hi == 0xFFFF) end = kEndOpen;
@@ -1023,9 +1044,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
         // Chunks until the next poll.  In a launch of few instances (P.eager: at least kEagerWarps
         // warps for each) and while more than half of the warps wait, a warp polls after every chunk and
         // hands out up to kEagerShares pieces at once, and so do the warps it gives work to: the time
-        // until the chip is busy is the chain of first donations (12 staged searches of the combination
-        // step's configurations: 9.5 ms at 16 chunks per poll, 5.9 ms so).  With more instances it
-        // would only cut the work into smaller pieces (1,000 searches: 2 % slower at 4 chunks per poll).
+        // until the chip is busy is the chain of first donations.  Polling after 16 chunks -> eagerly:
+        // full sortings of 4..6 3-cycles one by one 2.54 -> 0.55 ms, 64 in a launch 12.5 -> 7.4 ms;
+        // partial searches of 8..10 3-cycles 0.51 -> 0.12 ms, 64 in a launch 6.8 -> 1.9 ms.  Past the
+        // bound (74 instances) full sortings would still gain (125 in a launch 16.4 -> 11.5 ms, 1,000
+        // 67 -> 62), but 500 partial searches take the same time (36.5 -> 40 ms) and a batch of 400 came
+        // back with shorter sequences (450 moves instead of 760), so the bound keeps to the launches
+        // where both kinds gain.
         int poll = P.eager && (kind == 2 || (S.staging[3] & kTaskEager)) ? 1 : P.pollInterval;
         while (outcome == 0) {
             if (setup) {
