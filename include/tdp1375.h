@@ -126,10 +126,10 @@ int tdp_last_stats(int slot, tdp_stats *out);
 
 typedef struct tdp_engine_config {
     int32_t blocks_per_sm;   /* 0 = occupancy maximum */
-    int32_t poll_interval;   /* chunks between flag polls / donation checks; 16 (default) leaves it to
-                                the launch: 128 when every instance stops at its first sequence and
-                                there are three for every eight warps (under a learned order one for
-                                every warp), else 16 */
+    int32_t poll_interval;   /* chunks between flag polls / donation checks; 16 (default) lets the
+                                launch go over to 128 after 16 ms when every instance stops at its
+                                first sequence and there are three for every eight warps (under a
+                                learned order one for every warp) */
     int32_t tight_bound;     /* 1 = verdict-preserving strengthened prune, 0 = reference prune only */
     int32_t task_capacity;   /* read-only: warp mailboxes for work donation (sized from the queue budget) */
     double time_limit_s;     /* device deadline per launch */

@@ -143,6 +143,7 @@ struct EngineParams {
     InstanceOut *out;
     int count;
     int pollInterval;
+    int widePoll;             // > 0: chunks between two polls once the launch has run for 16 ms
     const RuleTable *rules;
     const uint32_t *triples;  // lexicographic (i,j,k) per n at offset combinations4(n)
     void *table;

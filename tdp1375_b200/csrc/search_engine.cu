@@ -293,10 +293,10 @@ int SearchSlot::stage(const tdp_instance *instances, int count, float minRate, s
     return 0;
 }
 
-// Chunks between two polls of a busy warp when the configuration leaves it to the launch.  A
-// search that must be exhausted visits the same nodes however it is shared, so it is shared
-// early.  One that stops at its first sequence visits the more nodes the wider its front, and the
-// nearer the instances come to one per warp, the less sharing buys.  Times on one B200 (4,736
+// Longer interval between two polls (or 0) when the configuration leaves it to the launch.  A search
+// that must be exhausted visits the same nodes however it is shared, so it is shared early, after
+// 16 chunks.  One that stops at its first sequence visits the more nodes the wider its front, and
+// the nearer the instances come to one per warp, the less sharing buys.  Times on one B200 (4,736
 // warps), partial mode, at 16 / 64 / 128 chunks per poll, by instances in a launch:
 //   20,000 of 8..10 3-cycles    1,000  1,377 / 1,372 / 1,445 ms    2,000  2,349 / 1,994 / 1,943
 //                               3,000  2,477 / 2,084 / 1,958      10,000  3,652 / 3,354 / 3,185
@@ -306,12 +306,15 @@ int SearchSlot::stage(const tdp_instance *instances, int count, float minRate, s
 //   (3..10)                     5,000  114 / 113 / 114             8,000  213 / 196 / 189
 // (32 lies between 16 and 64, 256 is no better than 128; nodes in proportion to the times).
 // Searches under the learned order end sooner, so few of them are left for the waiting warps: the
-// line is where every warp has one.  A cap on the instances in flight does not move it: 100,000
-// uneven instances at 8 warps each 1,059 / 919 / 807 ms.  Full sortings of 4..6 3-cycles, 1,000 in
-// a launch: 268 ms per 4,000 at 16, 322 at 64.
+// line is where every warp has one.  Launches of a few milliseconds are all tail and want early
+// sharing (6,000 of 3..6 3-cycles: 6.1 ms at 16, 12.3 at 128), so the longer interval starts after
+// 16 ms of a launch: 6.2 ms, and 1,961 / 1,978 / 3,267 ms for 2,000 / 3,000 / 10,000 of 8..10 in a
+// launch.  A cap on the instances in flight does not move the line: 100,000 uneven instances at 8
+// warps each 1,059 / 919 / 807 ms.  Full sortings of 4..6 3-cycles, 1,000 in a launch: 268 ms per
+// 4,000 at 16, 322 at 64.
 constexpr int kDefaultPoll = 16, kWidePoll = 128;
-static int launch_poll(int64_t count, int64_t warps, bool exhaustive, bool ordered) {
-    return !exhaustive && (ordered ? count >= warps : 8 * count >= 3 * warps) ? kWidePoll : kDefaultPoll;
+static int wide_poll(int64_t count, int64_t warps, bool exhaustive, bool ordered) {
+    return !exhaustive && (ordered ? count >= warps : 8 * count >= 3 * warps) ? kWidePoll : 0;
 }
 
 void SearchSlot::launchClass(int cls, int offset, int count) {
@@ -359,7 +362,7 @@ void SearchSlot::launchClass(int cls, int offset, int count) {
     if (P.maxInFlight >= count) P.maxInFlight = 0;
     P.pollInterval = cfg_.poll_interval;
     if (P.pollInterval == kDefaultPoll)
-        P.pollInterval = launch_poll(count, (int64_t)grid * dev::kWarpsPerBlock, exhaustive_[cls], P.order != nullptr);
+        P.widePoll = wide_poll(count, (int64_t)grid * dev::kWarpsPerBlock, exhaustive_[cls], P.order != nullptr);
     // the generation word is read from hGen_[cls], which runStaged set before this run
     const int resetBlocks = std::min(numSMs_, std::max(16, (count * (int)(sizeof(InstanceOut) / 16) + 255) / 256));
     dev::reset_kernel<<<resetBlocks, 256, 0, stream_>>>(dCtl_, dOut_ + offset, count, dDone_, dMail_, mailboxes_, dRing_,

@@ -49,6 +49,7 @@ constexpr int kWarpsPerBlock = 8;
 constexpr int kSpinLimit = 1 << 20;
 constexpr uint32_t kFlagCycles = 2000;
 constexpr int kLooks = 32;  // at some 0.7 us each
+constexpr unsigned long long kWideAfterNs = 16000000;
 
 template <int NW>
 struct KeyTraits;
@@ -1088,7 +1089,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                         const int cancelFlag = ld_relaxed_s32(P.cancel);
                         const int state = ld_relaxed_s32(&P.out[inst].state);
                         const int idle = ld_relaxed_s32(&ctl->idle);
-                        const bool late = global_time_ns() > deadline;
+                        const unsigned long long now = global_time_ns();
+                        const bool late = now > deadline;
                         if (stopFlag | cancelFlag) {
                             act = 2;
                         } else if (late) {
@@ -1101,10 +1103,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                             act = 3;
                         }
                         if (P.eager && 2 * idle > (int)(gridDim.x * kWarpsPerBlock)) act |= 4;
+                        if (P.widePoll && now + P.timeLimitNs > deadline + kWideAfterNs) act |= 8;
                     }
                     act = __shfl_sync(kFull, act, 0);
                     const bool eager = act & 4;
-                    poll = eager ? 1 : P.pollInterval;
+                    poll = eager ? 1 : (act & 8) ? P.widePoll : P.pollInterval;
                     act &= 3;
                     if (act == 1 || act == 2) {
                         outcome = act;
