@@ -770,6 +770,8 @@ struct WarpShared {
     uint32_t cycles[NW == 1 ? 1 : 128];          // sparse_setup's scratch
     uint64_t rules[32];                       // success (0..15) and expansion (16..31) tables of the instance
     unsigned long long taskNodes, taskChildren;  // counters of the task in hand
+    int interval;                                // chunks between two polls (carried in the poll's
+                                                 // shuffle it made eager launches 2 % slower)
     int firstInstance;                           // taken when the block started; count or more: none (left)
     int rank1;                                   // root-order rank of the current first-level node (-1: none)
     uint32_t staging[52];
@@ -844,7 +846,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
     __syncthreads();
     const uint32_t gw = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const int busy = max(0, min(P.count - blockFirst, kWarpsPerBlock));  // (of no meaning when blockFirst < 0)
-    if (lane == 0) S.firstInstance = blockFirst < 0 ? P.count : blockFirst + own;
+    if (lane == 0) {
+        S.firstInstance = blockFirst < 0 ? P.count : blockFirst + own;
+        S.interval = P.pollInterval;
+    }
     bool registered = blockFirst >= 0 && own >= busy;
     if (registered && own == kWarpsPerBlock - 1) ring_enter_block(P, busy, lane);
     int backoff = 64;
@@ -1103,11 +1108,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, NW == 1 ? 4 : 2) search_e
                             act = 3;
                         }
                         if (P.eager && 2 * idle > (int)(gridDim.x * kWarpsPerBlock)) act |= 4;
-                        if (P.widePoll && now + P.timeLimitNs > deadline + kWideAfterNs) act |= 8;
+                        if (P.widePoll && now + P.timeLimitNs > deadline + kWideAfterNs) S.interval = P.widePoll;
                     }
                     act = __shfl_sync(kFull, act, 0);
+                    __syncwarp();  // every lane reads the interval that lane 0 may just have written
                     const bool eager = act & 4;
-                    poll = eager ? 1 : (act & 8) ? P.widePoll : P.pollInterval;
+                    poll = eager ? 1 : S.interval;
                     act &= 3;
                     if (act == 1 || act == 2) {
                         outcome = act;
