@@ -37,7 +37,6 @@
 // Spans of 256 / 1,024 triples 23.2 / 23.1 us, blocks of 128 threads 21.8 us.
 #include <cuda_runtime.h>
 
-#include <algorithm>
 #include <cstdint>
 #include <string>
 

@@ -13,7 +13,7 @@ namespace mlp {
 constexpr int kFeatures = 1088;     // 32x32 adjacency bits + 64-bin cycle-length histogram
 constexpr int kHidden = 256;
 constexpr int kTriples = 4960;        // C(32,3)
-constexpr int kTriplesPadded = 5120;  // 20 tiles of 256
+constexpr int kTriplesPadded = 5120;  // 40 tiles of 128
 
 struct GemmParams {
     int M, N, K;

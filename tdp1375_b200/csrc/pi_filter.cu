@@ -235,11 +235,11 @@ __global__ void __launch_bounds__(kThreads) pi_filter_write_kernel(const FilterA
 // The neighbours of a warp share most of their codes, so the table reads are broadcasts.
 // Deciding one candidate at a time (next-permutation steps, 32 ranks per thread) cost some
 // hundred instructions for each and twice, as the writing pass decided them again: n = 12
-// with a 7-cycle took 1,057 us on the device and takes 51 us (count, scan and write; 40 M
+// with a 7-cycle took 1,057 us on the device and takes 51 us (count and write; 40 M
 // candidates, bound by instruction issue), n = 9 took 117 us and takes 20 us (two launches'
-// latency).  With the workspaces kept (below) the whole calls went from 3.1 ms to 0.14 ms and
-// from 1.0 ms to 64 us; with 831,600 rows (10 MB) the rest of a call, 0.55 ms, is their copy
-// to the caller's pageable buffer.
+// latency).  With the workspaces kept (below) the whole calls went from 2.3 ms to 91 us and
+// from 0.8 ms to 46 us (repeated calls; the first on new inputs 140 and 73 us); with 831,600 rows
+// (10 MB) the rest of a call, 0.55 ms, is their copy to the caller's pageable buffer.
 constexpr int kPackedMaxN = 16;
 constexpr int kTail = 5;
 constexpr int kTailRanks = 120;

@@ -3,9 +3,10 @@
 The model scores the C(32,3) = 4960 position triples (i<j<k) of a configuration with
 n <= 32 symbols: 1088 inputs (32x32 adjacency of spi in pi-position coordinates + a 64-bin
 cycle-length histogram), three hidden layers of 256 (ReLU), 4960 outputs.  All matrix
-products run in the library's tcgen05 GEMM (``tdp_mlp_gemm``); torch only holds device
-memory.  Training pairs are (state, next move) along the solutions the plain search finds;
-the loss is softmax cross-entropy over the triples valid for the state's n.
+products run in the library's tcgen05 GEMM: the forward pass through ``tdp_mlp_gemm``, a
+training step as one call (``tdp_mlp_train_step``); torch only holds device memory.  Training
+pairs are (state, next move) along the solutions the plain search finds; the loss is softmax
+cross-entropy over the triples valid for the state's n.
 
 Installing the model on a slot makes the batched search expand every instance's root
 children in descending score order.  Ordering permutes children only, so verdicts do not

@@ -1,7 +1,7 @@
 """Launches of many searches that stop at their first sequence share work late: handing out pieces
 of a search early widens its front and with it the nodes expanded before the sequence is met (3,000
 searches of 8..10 3-cycles in a launch: 1,182 M nodes per 20,000 searches at 16 chunks per poll,
-937 M by default)."""
+about 960 M by default)."""
 import numpy as np
 import pytest
 
